@@ -27,6 +27,7 @@
 #include "batch.h"
 #include "rc_host.h"
 #include "tune_cache.h"
+#include "tree_build.h"
 
 using orn::RenderLaunch;
 using orn::SceneDev;
@@ -292,57 +293,6 @@ int build_lights(orn_context* ctx, const orn_scene_blob* b) {
     ctx->d_light_cdf = dc;
     ctx->d_light_material = dm;
     return ORN_OK;
-}
-
-// Re-lays the reference's BvhNode arrays into the kernel's node array.
-void relayout_nodes(const orn_scene_blob* b, std::vector<float4>* out) {
-    const uint32_t T = b->tlas_nodes_len, B = b->blas_nodes_len;
-    out->assign((size_t)(T + B) * 4, make_float4(0, 0, 0, 0));
-    auto u2f = [](uint32_t u) { float f; std::memcpy(&f, &u, 4); return f; };
-    // reference to node `i` of the TLAS (blas=false) or BLAS, with its type
-    auto ref = [&](uint32_t i, bool blas) -> uint32_t {
-        const orn_bvh_node& c = blas ? b->blas_nodes[i] : b->tlas_nodes[i];
-        return ((blas ? T : 0u) + i) | (c.node_type << 30);
-    };
-    auto put = [&](size_t idx, const orn_bvh_node& n, uint32_t child_offset) {
-        float4* o = out->data() + idx * 4;
-        const float* a = n.left_aabb_min_or_v0;
-        const float* bb = n.left_aabb_max_or_v1;
-        const float* c = n.right_aabb_min_or_v2;
-        const float* e = n.right_aabb_max_or_v3;
-        switch (n.node_type) {
-            case ORN_NODE_INTERNAL:
-                o[0] = make_float4(a[0], a[1], a[2], u2f(ref(n.left_or_custom_id, child_offset != 0)));
-                o[1] = make_float4(bb[0], bb[1], bb[2], u2f(ref(n.right_or_material_index, child_offset != 0)));
-                o[2] = make_float4(c[0], c[1], c[2], u2f(ORN_NODE_INTERNAL));
-                o[3] = make_float4(e[0], e[1], e[2], 0.0f);
-                break;
-            case ORN_NODE_TRIANGLE: {
-                // the vertices as given, so triangles sharing an edge see the
-                // same floats (the watertight test relies on it), and the two
-                // edges the reference's test subtracts on the fly
-                // (bvh.hip.h:81-82) — the same single-precision subtractions
-                const float e1[3] = {bb[0] - a[0], bb[1] - a[1], bb[2] - a[2]};
-                const float e2[3] = {c[0] - a[0], c[1] - a[1], c[2] - a[2]};
-                o[0] = make_float4(a[0], a[1], a[2], u2f(n.left_or_custom_id));
-                o[1] = make_float4(bb[0], bb[1], bb[2], e2[0]);
-                o[2] = make_float4(c[0], c[1], c[2], e2[1]);
-                o[3] = make_float4(e1[0], e1[1], e1[2], e2[2]);
-                break;
-            }
-            default: {  // sphere / mesh leaf: inverse rows 0..2 inline
-                const float* m = b->transforms + (size_t)n.transform_id * 2 * 16;
-                o[0] = make_float4(m[0], m[1], m[2], m[3]);
-                o[1] = make_float4(m[4], m[5], m[6], m[7]);
-                o[2] = make_float4(m[8], m[9], m[10], u2f(n.node_type));
-                uint32_t root = n.node_type == ORN_NODE_MESH ? ref(n.left_or_custom_id, true) : 0u;
-                o[3] = make_float4(m[11], u2f(n.right_or_material_index), u2f(n.transform_id), u2f(root));
-                break;
-            }
-        }
-    };
-    for (uint32_t i = 0; i < T; ++i) put(i, b->tlas_nodes[i], 0);
-    for (uint32_t i = 0; i < B; ++i) put((size_t)T + i, b->blas_nodes[i], T);
 }
 
 int ensure_target(orn_context* ctx) {
@@ -748,11 +698,7 @@ int orn_create(const orn_scene_blob* blob, int device, orn_context** out) {
         ORN_CUDA(ctx, cudaEventCreateWithFlags(&ctx->na_done, cudaEventDisableTiming));
         ORN_CUDA(ctx, cudaMalloc(&ctx->d_counters, ORN_COUNTER_COUNT * sizeof(unsigned long long)));
         ORN_CUDA(ctx, cudaMemset(ctx->d_counters, 0, ORN_COUNTER_COUNT * sizeof(unsigned long long)));
-        std::vector<float4> nodes;
-        relayout_nodes(blob, &nodes);
-        float4* d_nodes = nullptr;
-        int s = upload(ctx, nodes.data(), nodes.size(), &d_nodes);
-        if (s) return s;
+        int s;
         float4* d_x = nullptr;
         if ((s = upload(ctx, (const float4*)blob->transforms, (size_t)blob->transforms_len * 4, &d_x))) return s;
         float4* d_n = nullptr;
@@ -791,26 +737,15 @@ int orn_create(const orn_scene_blob* blob, int device, orn_context** out) {
         }
         TexDesc* d_t = nullptr;
         if ((s = upload(ctx, descs.data(), descs.size(), &d_t))) return s;
-        ctx->scene.nodes = d_nodes;
+        orn::NodeFacts facts{};
+        ORN_CUDA(ctx, orn::build_scene_trees(blob, d_x, &ctx->scene, &facts, &ctx->scene_allocs, ctx->stream));
         ctx->scene.tlas_len = blob->tlas_nodes_len;
         ctx->scene.node_count = blob->tlas_nodes_len + blob->blas_nodes_len;
         ctx->scene.root_ref = (blob->tlas_nodes_len - 1) |
                               (blob->tlas_nodes[blob->tlas_nodes_len - 1].node_type << 30);
         // The FMNMX slab test needs every internal-node bound finite and
         // below 1e30 in magnitude (pt_device.cuh, aabb_hit_fast).
-        bool huge = false;
-        auto check_bounds = [&](const orn_bvh_node* nodes, uint32_t n) {
-            for (uint32_t i = 0; i < n && !huge; ++i) {
-                if (nodes[i].node_type != ORN_NODE_INTERNAL) continue;
-                const float* f[4] = {nodes[i].left_aabb_min_or_v0, nodes[i].left_aabb_max_or_v1,
-                                     nodes[i].right_aabb_min_or_v2, nodes[i].right_aabb_max_or_v3};
-                for (int k = 0; k < 4; ++k)
-                    for (int j = 0; j < 3; ++j)
-                        if (!(std::fabs(f[k][j]) < 1e30f)) huge = true;
-            }
-        };
-        check_bounds(blob->tlas_nodes, blob->tlas_nodes_len);
-        check_bounds(blob->blas_nodes, blob->blas_nodes_len);
+        bool huge = facts.huge != 0;
         for (uint32_t i = 0; i < blob->tlas_nodes_len; ++i) {
             const orn_bvh_node& n = blob->tlas_nodes[i];
             const float* f[4] = {n.left_aabb_min_or_v0, n.left_aabb_max_or_v1, n.right_aabb_min_or_v2,

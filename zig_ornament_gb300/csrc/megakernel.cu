@@ -15,11 +15,14 @@
 #include "pt_kernels.h"
 #include "pt_device.cuh"
 #include "pt_machine.cuh"
+#include "pt_near.cuh"
 #include "qmc.cuh"
+
+#include <type_traits>
 
 namespace orn {
 
-enum LaneMode { LANE_IDLE = 0, LANE_TRAVERSE = 1, LANE_SHADE = 2, LANE_DONE = 3 };
+enum LaneMode { LANE_IDLE = 0, LANE_TRAVERSE = 1, LANE_SHADE = 2, LANE_DONE = 3, LANE_START = 4 };
 
 
 // Per-pixel accumulation: FP32 RGBA as the reference keeps it
@@ -76,11 +79,13 @@ template <> struct Accum<true> {
 #ifndef ORN_CACHE_MIN_BLOCKS
 #define ORN_CACHE_MIN_BLOCKS 7
 #endif
-template <int SEM, int MATH, bool COUNT, bool FAST, bool F64 = false, bool CACHE = false, bool SOBOL = false>
-__global__ void __launch_bounds__(kMegaBlock, CACHE ? ORN_CACHE_MIN_BLOCKS : kMegaMinBlocks)
+template <int SEM, int MATH, bool COUNT, bool FAST, bool F64 = false, bool CACHE = false, bool SOBOL = false,
+          bool NEAR = false>
+__global__ void __launch_bounds__(kMegaBlock, CACHE ? ORN_CACHE_MIN_BLOCKS : (NEAR ? kNearMinBlocks : kMegaMinBlocks))
 mega_kernel(RenderLaunch p) {
+    static_assert(!NEAR || (FAST && !COUNT && !CACHE), "near-first trees: the plain kernel with the FMNMX slab test");
     __shared__ uint32_t sstack[kSmemStack * kMegaBlock];
-    TravStack<kSmemStack> stack;
+    TravStack<kSmemStack, NEAR ? kNearStackWords : kStackSize> stack;
     stack.sstack = sstack + threadIdx.x;
     stack.sstride = kMegaBlock;
     const unsigned kFull = 0xffffffffu;
@@ -103,7 +108,7 @@ mega_kernel(RenderLaunch p) {
     f3 ro = mk(0.0f, 0.0f, 0.0f), rd = ro, color = ro;
     HitRec h;
     h.t = 0.0f; h.material = 0; h.type = 0; h.inv = 0; h.tri = 0; h.u = 0.0f; h.v = 0.0f;
-    Walker w;
+    std::conditional_t<NEAR, NearWalker, Walker> w;
     VisitCount vc = {0, 0, 0, 0, 0};
     SampleCount scn = {0, 0, 0, 0};
     uint32_t err = 0;
@@ -185,9 +190,14 @@ mega_kernel(RenderLaunch p) {
     };
 
     for (;;) {
-        // Hand out pixels to idle lanes: one atomic per warp.
-        unsigned idle = __ballot_sync(kFull, mode == LANE_IDLE);
-        if (idle != 0u && !exhausted) {
+        // Lanes whose sample is complete start the next one (or complete the
+        // pixel), and idle lanes are handed pixels, one atomic per warp, until
+        // every lane has a ray or the pixels run out.  (start_samples is long:
+        // one copy of it, for the instruction cache.)
+        for (;;) {
+            if (mode == LANE_START) mode = start_samples();
+            const unsigned idle = __ballot_sync(kFull, mode == LANE_IDLE);
+            if (idle == 0u || exhausted) break;
             const unsigned leader = __ffs(idle) - 1u;
             const unsigned n = __popc(idle);
             uint32_t base = 0;
@@ -212,7 +222,7 @@ mega_kernel(RenderLaunch p) {
                         rng.state = p.rng[gid];
                         acc.load(p, gid, ci0);
                     }
-                    mode = start_samples();
+                    mode = LANE_START;
                 }
             }
         }
@@ -229,17 +239,28 @@ mega_kernel(RenderLaunch p) {
             // slower: the extra ballots cost more than the waiting lanes.)
             constexpr bool kPerStep = COUNT || CACHE || F64;
             uint32_t s = 0;
+            if constexpr (NEAR) {
 #pragma unroll 1
-            while (s < (uint32_t)kStepsPerIteration) {
-                ++s;
-                if (!walker_step<COUNT, kSmemStack, FAST, CACHE, kPerStep>(w, p.scene, ro, rd, p.cp.ray_cast_epsilon,
-                                                                           &h, stack, &vc, &err)) {
-                    mode = LANE_SHADE;
-                    break;
+                while (s < (uint32_t)kNearSteps) {
+                    ++s;
+                    if (!near_step(w, p.scene, ro, rd, p.cp.ray_cast_epsilon, stack)) {
+                        mode = LANE_SHADE;
+                        break;
+                    }
                 }
+            } else {
+#pragma unroll 1
+                while (s < (uint32_t)kStepsPerIteration) {
+                    ++s;
+                    if (!walker_step<COUNT, kSmemStack, FAST, CACHE, kPerStep>(w, p.scene, ro, rd, p.cp.ray_cast_epsilon,
+                                                                               &h, stack, &vc, &err)) {
+                        mode = LANE_SHADE;
+                        break;
+                    }
+                }
+                if (!kPerStep && mode == LANE_TRAVERSE && !walker_account_round(w, s, &err)) mode = LANE_SHADE;
             }
             steps += s;
-            if (!kPerStep && mode == LANE_TRAVERSE && !walker_account_round(w, s, &err)) mode = LANE_SHADE;
         }
 
         const unsigned ready = __ballot_sync(kFull, mode == LANE_SHADE);
@@ -283,14 +304,10 @@ mega_kernel(RenderLaunch p) {
                             // unless the previous vertex sampled this emitter directly
                             // (shade_geom's emission, computed here: a second inlined
                             // copy of shade_geom cost instruction-cache misses)
-                            const uint32_t etex = bits(ma.w);
-                            const bool etex_on = SEM == SEM_WGSL
-                                                     ? (etex < p.cp.textures_count && etex < p.scene.textures_len)
-                                                     : etex < p.scene.textures_len;
-                            f3 em = mk(0.0f, 0.0f, 0.0f);
-                            if (mtype == ORN_DIFFUSE_LIGHT)
-                                em = etex_on ? tex_sample(p.scene.textures[etex], g.hu, g.hv, SEM == SEM_WGSL)
-                                             : mk(ma.x, ma.y, ma.z);
+                            bool textured;
+                            const f3 em = mtype == ORN_DIFFUSE_LIGHT
+                                              ? surface_color<SEM, MATH_PORTABLE>(p.scene, p.cp, h, g, ma, &textured)
+                                              : mk(0.0f, 0.0f, 0.0f);
                             f3 c2 = mul(color, em);
                             const bool sampled = nee_prev && h.type == ORN_NODE_MESH &&
                                                  __ldg(p.cache.light_material + h.material) != 0u;
@@ -311,12 +328,8 @@ mega_kernel(RenderLaunch p) {
                             const bool rough = mtype == ORN_LAMBERTIAN || (mtype == ORN_METAL && mb.x >= kCacheMinFuzz);
                             // the surface colour (lambertian and metal attenuation)
                             auto surface_att = [&]() -> f3 {
-                                const uint32_t tex_id = bits(ma.w);
-                                const bool use_tex = SEM == SEM_WGSL
-                                                         ? (tex_id < p.cp.textures_count && tex_id < p.scene.textures_len)
-                                                         : tex_id < p.scene.textures_len;
-                                return use_tex ? tex_sample(p.scene.textures[tex_id], g.hu, g.hv, SEM == SEM_WGSL)
-                                               : mk(ma.x, ma.y, ma.z);
+                                bool textured;
+                                return surface_color<SEM, MATH_PORTABLE>(p.scene, p.cp, h, g, ma, &textured);
                             };
                             bool at_cache = false;
                             f3 aclamp = mk(1.0f, 1.0f, 1.0f);
@@ -506,11 +519,13 @@ mega_kernel(RenderLaunch p) {
                         }
                         add_sample(c);
                         ++k;
-                        mode = start_samples();
+                        mode = LANE_START;
                     }
                 } else {
-                    bool cont;
-                    if (!w.any) {
+                    bool cont, any;
+                    if constexpr (NEAR) any = near_finish(w, p.scene, &h);
+                    else any = w.any;
+                    if (!any) {
                         if (err) color = mk(0.0f, 0.0f, 0.0f);
                         else color = sky_color(color, rd);
                         cont = false;
@@ -524,7 +539,7 @@ mega_kernel(RenderLaunch p) {
                     } else {
                         acc.add(ci0 + (float)k, color);
                         ++k;
-                        mode = start_samples();
+                        mode = LANE_START;
                     }
                 }
             }
@@ -547,7 +562,10 @@ mega_kernel(RenderLaunch p) {
     }
 }
 
-// Bvh::hit on a ray list (parity / debugging entry point).
+// Bvh::hit on a ray list (parity / debugging entry point).  NEAR: on the
+// near-first trees (rays that their traversal does not take, and every ray when
+// visits are asked for, walk the reference's tree).
+template <bool NEAR>
 __global__ void __launch_bounds__(128)
 trace_rays_kernel(SceneDev sc, float t_min, const float* __restrict__ rays, size_t count,
                   orn_hit* __restrict__ hits, uint32_t* __restrict__ visits, uint32_t* error) {
@@ -560,7 +578,19 @@ trace_rays_kernel(SceneDev sc, float t_min, const float* __restrict__ rays, size
     h.t = 0.0f; h.material = 0; h.type = 0; h.inv = 0; h.tri = 0; h.u = 0.0f; h.v = 0.0f;
     VisitCount vc = {0, 0, 0, 0, 0};
     uint32_t err = 0;
-    bool any = trace_ray<true, kSmemStack>(sc, ro, rd, t_min, &h, &vc, &err, sstack + threadIdx.x, 128);
+    bool any;
+    if (NEAR && slab_safe(ro)) {
+        NearStack<kSmemStack> stack;
+        stack.sstack = sstack + threadIdx.x;
+        stack.sstride = 128;
+        NearWalker w;
+        walker_begin(w, sc, ro, rd);
+#pragma unroll 1
+        while (near_step(w, sc, ro, rd, t_min, stack)) {}
+        any = near_finish(w, sc, &h);
+    } else {
+        any = trace_ray<true, kSmemStack>(sc, ro, rd, t_min, &h, &vc, &err, sstack + threadIdx.x, 128);
+    }
     orn_hit o;
     o.hit = any ? 1u : 0u;
     o.t = any ? h.t : 0.0f;
@@ -654,7 +684,8 @@ cudaError_t launch_relmse(const float4* acc, const double* acc64, const double* 
 // ---- host-side launchers -----------------------------------------------------
 // Persistent grid: as many blocks as fit on the device at once (never more
 // than the pixels need).
-template <int SEM, int MATH, bool COUNT, bool FAST, bool F64 = false, bool CACHE = false, bool SOBOL = false>
+template <int SEM, int MATH, bool COUNT, bool FAST, bool F64 = false, bool CACHE = false, bool SOBOL = false,
+          bool NEAR = false>
 static cudaError_t launch_mega_tt(const RenderLaunch& p, cudaStream_t s) {
     static int blocks_per_sm = 0, sms = 0;
     if (blocks_per_sm == 0) {
@@ -663,10 +694,10 @@ static cudaError_t launch_mega_tt(const RenderLaunch& p, cudaStream_t s) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 #ifdef ORN_MEGA_CARVEOUT
         // shared-memory share of the unified L1/shared space, in percent
-        cudaFuncSetAttribute(mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL>,
+        cudaFuncSetAttribute(mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR>,
                              cudaFuncAttributePreferredSharedMemoryCarveout, ORN_MEGA_CARVEOUT);
 #endif
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL>,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR>,
                                                       kMegaBlock, 0);
         if (blocks_per_sm < 1) blocks_per_sm = 1;
     }
@@ -676,7 +707,7 @@ static cudaError_t launch_mega_tt(const RenderLaunch& p, cudaStream_t s) {
     if (need < grid) grid = need;
     cudaError_t e = cudaMemsetAsync(p.work_counter, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL><<<grid, kMegaBlock, 0, s>>>(p);
+    mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR><<<grid, kMegaBlock, 0, s>>>(p);
     return cudaGetLastError();
 }
 
@@ -698,6 +729,8 @@ cudaError_t launch_mega_cached(const RenderLaunch& p, int semantics, bool fast, 
 
 template <int SEM>
 static cudaError_t launch_mega_t(const RenderLaunch& p, bool count, bool fast, cudaStream_t s) {
+    if (fast && !count && p.scene.near)
+        return launch_mega_tt<SEM, MATH_PORTABLE, false, true, false, false, false, true>(p, s);
     if (fast) return count ? launch_mega_tt<SEM, MATH_PORTABLE, true, true>(p, s)
                            : launch_mega_tt<SEM, MATH_PORTABLE, false, true>(p, s);
     return count ? launch_mega_tt<SEM, MATH_PORTABLE, true, false>(p, s)
@@ -705,6 +738,9 @@ static cudaError_t launch_mega_t(const RenderLaunch& p, bool count, bool fast, c
 }
 
 cudaError_t launch_mega_f64(const RenderLaunch& p, int semantics, bool fast, cudaStream_t s) {
+    if (fast && p.scene.near)
+        return semantics == SEM_WGSL ? launch_mega_tt<SEM_WGSL, MATH_PORTABLE, false, true, true, false, false, true>(p, s)
+                                     : launch_mega_tt<SEM_HIP, MATH_PORTABLE, false, true, true, false, false, true>(p, s);
     if (semantics == SEM_WGSL)
         return fast ? launch_mega_tt<SEM_WGSL, MATH_PORTABLE, false, true, true>(p, s)
                     : launch_mega_tt<SEM_WGSL, MATH_PORTABLE, false, false, true>(p, s);
@@ -724,7 +760,9 @@ cudaError_t launch_trace_rays(const SceneDev& sc, float t_min, const float* rays
                               orn_hit* hits, uint32_t* visits, uint32_t* error, cudaStream_t s) {
     if (count == 0) return cudaSuccess;
     size_t blocks = (count + 127) / 128;
-    trace_rays_kernel<<<(unsigned)blocks, 128, 0, s>>>(sc, t_min, rays, count, hits, visits, error);
+    if (sc.near && !sc.exact_slabs && !visits)
+        trace_rays_kernel<true><<<(unsigned)blocks, 128, 0, s>>>(sc, t_min, rays, count, hits, visits, error);
+    else trace_rays_kernel<false><<<(unsigned)blocks, 128, 0, s>>>(sc, t_min, rays, count, hits, visits, error);
     return cudaGetLastError();
 }
 

@@ -301,19 +301,29 @@ struct VisitCount {
 // ERR_* bits when the ray is abandoned (the result is then a miss).
 // Traversal stack: the first SS entries live in shared memory (entry i of
 // this thread at sstack[i * sstride], so a warp's accesses hit 32 distinct
-// banks), deeper entries spill to a per-thread local array; the total depth
-// is the reference's 64.
-template <int SS>
+// banks), deeper entries spill to a per-thread local array; the total size
+// is the reference's 64 entries unless SIZE says otherwise.
+template <int SS, int SIZE = kStackSize>
 struct TravStack {
     uint32_t* sstack;
     int sstride;
-    uint32_t lstack[kStackSize - SS > 0 ? kStackSize - SS : 1];
+    uint32_t lstack[SIZE - SS > 0 ? SIZE - SS : 1];
     __device__ __forceinline__ void put(int i, uint32_t v) {
-        if (SS >= kStackSize || i < SS) sstack[i * sstride] = v;
+        if (SS >= SIZE || i < SS) sstack[i * sstride] = v;
         else lstack[i - SS] = v;
     }
+    // a pair of words at an even place (SS is even)
+    __device__ __forceinline__ void put2(int i, uint32_t a, uint32_t b) {
+        if (SS >= SIZE || i < SS) {
+            sstack[i * sstride] = a;
+            sstack[(i + 1) * sstride] = b;
+        } else {
+            lstack[i - SS] = a;
+            lstack[i + 1 - SS] = b;
+        }
+    }
     __device__ __forceinline__ uint32_t get(int i) const {
-        if (SS >= kStackSize || i < SS) return sstack[i * sstride];
+        if (SS >= SIZE || i < SS) return sstack[i * sstride];
         return lstack[i - SS];
     }
 };
@@ -530,55 +540,79 @@ __device__ __forceinline__ f3 sky_color(f3 color, f3 rd) {
 }
 
 // Surface point of a hit (pathtracer.hip.cpp:95-131): position, the normal
-// facing the incoming ray, the side, and the texture coordinates.
+// facing the incoming ray, and the side.
 struct HitGeom {
     f3 hp, normal;
     bool front;
-    float hu, hv;
 };
 
+// Spheres and meshes differ in the vector that is normalised; the rest is
+// one piece of code, so a warp with both kinds of hits runs it once.
 template <int MATH, bool COUNT>
 __device__ __forceinline__ HitGeom hit_geometry(const SceneDev& sc, const HitRec& h, f3 ro, f3 rd, SampleCount* scn) {
-    typedef DevMath<MATH> M;
     HitGeom g;
     uint32_t transform_id = h.inv + 1u;
     g.hp = add(ro, scale(h.t, rd));
+    f3 n;
     if (h.type == ORN_NODE_SPHERE) {
         if (COUNT) scn->sphere_hits++;
         const float4* m = sc.xforms + 4 * (size_t)transform_id;
         f3 center = mk(dot4(ldg4(m), 0.0f, 0.0f, 0.0f, 1.0f), dot4(ldg4(m + 1), 0.0f, 0.0f, 0.0f, 1.0f),
                        dot4(ldg4(m + 2), 0.0f, 0.0f, 0.0f, 1.0f));
-        f3 on = normalize(sub(g.hp, center));
-        float theta = M::acos(-on.y);
-        float phi = M::atan2(-on.z, on.x) + 3.14159265358979f;
-        g.hu = phi / (2.0f * 3.14159265358979f);
-        g.hv = theta / 3.14159265358979f;
-        if (dot(rd, on) > 0.0f) { g.normal = neg(on); g.front = false; }
-        else { g.normal = on; g.front = true; }
+        n = sub(g.hp, center);
     } else {
         if (COUNT) scn->mesh_hits++;
         float4 n0 = ldg4(sc.normals + __ldg(sc.normal_indices + h.tri));
         float4 n1 = ldg4(sc.normals + __ldg(sc.normal_indices + h.tri + 1));
         float4 n2 = ldg4(sc.normals + __ldg(sc.normal_indices + h.tri + 2));
-        float2 t0 = __ldg(sc.uvs + __ldg(sc.uv_indices + h.tri));
-        float2 t1 = __ldg(sc.uvs + __ldg(sc.uv_indices + h.tri + 1));
-        float2 t2 = __ldg(sc.uvs + __ldg(sc.uv_indices + h.tri + 2));
         float w = 1.0f - h.u - h.v;
         float nx = w * n0.x + h.u * n1.x + h.v * n2.x;
         float ny = w * n0.y + h.u * n1.y + h.v * n2.y;
         float nz = w * n0.z + h.u * n1.z + h.v * n2.z;
-        g.hu = w * t0.x + h.u * t1.x + h.v * t2.x;
-        g.hv = w * t0.y + h.u * t1.y + h.v * t2.y;
         const float4* m = sc.xforms + 4 * (size_t)h.inv;
         float4 m0 = ldg4(m), m1 = ldg4(m + 1), m2 = ldg4(m + 2), m3 = ldg4(m + 3);
-        f3 tn = mk(m0.x * nx + m1.x * ny + m2.x * nz + m3.x * 0.0f,
-                   m0.y * nx + m1.y * ny + m2.y * nz + m3.y * 0.0f,
-                   m0.z * nx + m1.z * ny + m2.z * nz + m3.z * 0.0f);
-        f3 on = normalize(tn);
-        if (dot(rd, on) > 0.0f) { g.normal = neg(on); g.front = false; }
-        else { g.normal = on; g.front = true; }
+        n = mk(m0.x * nx + m1.x * ny + m2.x * nz + m3.x * 0.0f,
+               m0.y * nx + m1.y * ny + m2.y * nz + m3.y * 0.0f,
+               m0.z * nx + m1.z * ny + m2.z * nz + m3.z * 0.0f);
     }
+    const f3 on = normalize(n);
+    g.front = !(dot(rd, on) > 0.0f);
+    g.normal = g.front ? on : neg(on);
     return g;
+}
+
+// Texture coordinates of a hit, wanted only where the material has a texture:
+// a sphere's take an arc cosine and an arc tangent, a mesh's six dependent
+// loads.
+template <int MATH>
+__device__ __forceinline__ void hit_uv(const SceneDev& sc, const HitRec& h, const HitGeom& g, float* hu, float* hv) {
+    typedef DevMath<MATH> M;
+    if (h.type == ORN_NODE_SPHERE) {
+        const f3 on = g.front ? g.normal : neg(g.normal);
+        float theta = M::acos(-on.y);
+        float phi = M::atan2(-on.z, on.x) + 3.14159265358979f;
+        *hu = phi / (2.0f * 3.14159265358979f);
+        *hv = theta / 3.14159265358979f;
+    } else {
+        float2 t0 = __ldg(sc.uvs + __ldg(sc.uv_indices + h.tri));
+        float2 t1 = __ldg(sc.uvs + __ldg(sc.uv_indices + h.tri + 1));
+        float2 t2 = __ldg(sc.uvs + __ldg(sc.uv_indices + h.tri + 2));
+        float w = 1.0f - h.u - h.v;
+        *hu = w * t0.x + h.u * t1.x + h.v * t2.x;
+        *hv = w * t0.y + h.u * t1.y + h.v * t2.y;
+    }
+}
+
+// The surface colour of a hit: its texture's texel, or the plain albedo.
+template <int SEM, int MATH>
+__device__ __forceinline__ f3 surface_color(const SceneDev& sc, const orn_constant_params& cp, const HitRec& h,
+                                            const HitGeom& g, float4 ma, bool* textured) {
+    const uint32_t tex_id = bits(ma.w);
+    *textured = SEM == SEM_WGSL ? (tex_id < cp.textures_count && tex_id < sc.textures_len) : tex_id < sc.textures_len;
+    if (!*textured) return mk(ma.x, ma.y, ma.z);
+    float hu, hv;
+    hit_uv<MATH>(sc, h, g, &hu, &hv);
+    return tex_sample(sc.textures[tex_id], hu, hv, SEM == SEM_WGSL);
 }
 
 // Hit shading and material (pathtracer.hip.cpp:95-145, material.hip.h):
@@ -587,6 +621,11 @@ __device__ __forceinline__ HitGeom hit_geometry(const SceneDev& sc, const HitRec
 // `preset` (the cached renderer's Sobol sampler): a lambertian scatter takes
 // the polar and azimuthal uniforms of its in_unit_sphere direction from
 // (pu_theta, pu_phi) instead of the stream (the radius is normalised away).
+//
+// The materials run through one sequence — one power, one pair of sines and
+// cosines, one normalisation of the ray — with operands chosen per lane.  A
+// branch per material, each with its own copy, had a warp run them one after
+// the other, and the copies did not fit the instruction cache.
 template <int SEM, int MATH, bool COUNT>
 __device__ __forceinline__ bool shade_geom(const SceneDev& sc, const orn_constant_params& cp, Rng& rng,
                                            const HitRec& h, const HitGeom& g, f3* ro_io, f3* rd_io,
@@ -594,74 +633,70 @@ __device__ __forceinline__ bool shade_geom(const SceneDev& sc, const orn_constan
                                            float pu_theta = 0.0f, float pu_phi = 0.0f) {
     typedef DevMath<MATH> M;
     const f3 rd = *rd_io;
-    f3 color = *color_io;
-    const f3 hp = g.hp, normal = g.normal;
-    const bool front = g.front;
-    const float hu = g.hu, hv = g.hv;
-    float4 ma = ldg4(sc.materials + 2 * (size_t)h.material);
-    float4 mb = ldg4(sc.materials + 2 * (size_t)h.material + 1);
-    uint32_t mtype = bits(mb.z);
-    uint32_t tex_id = bits(ma.w);
-    bool use_tex = SEM == SEM_WGSL ? (tex_id < cp.textures_count && tex_id < sc.textures_len)
-                                   : tex_id < sc.textures_len;
-    if (mtype == ORN_LAMBERTIAN) {
-        f3 s;
-        if (preset) {
-            float st, ct, sp, cph;
-            DevMath<MATH>::sincos(3.14159265358979f * pu_theta, &st, &ct);
-            DevMath<MATH>::sincos(2.0f * 3.14159265358979f * pu_phi, &sp, &cph);
-            s = mk(st * cph, st * sp, ct);
+    const f3 color = *color_io, normal = g.normal;
+    const float4 ma = ldg4(sc.materials + 2 * (size_t)h.material);
+    const float4 mb = ldg4(sc.materials + 2 * (size_t)h.material + 1);
+    const uint32_t mtype = bits(mb.z);
+    const bool lambert = mtype == ORN_LAMBERTIAN, metal = mtype == ORN_METAL, glass = mtype == ORN_DIELECTRIC;
+    f3 att = mk(1.0f, 1.0f, 1.0f);
+    if (!glass && mtype <= ORN_DIFFUSE_LIGHT) {
+        bool textured;
+        att = surface_color<SEM, MATH>(sc, cp, h, g, ma, &textured);
+        if (COUNT && textured) scn->textured++;
+    }
+    if (mtype > ORN_DIELECTRIC) {
+        *color_io = mul(color, mtype == ORN_DIFFUSE_LIGHT ? att : mk(0.0f, 0.0f, 0.0f));
+        return false;
+    }
+    f3 ud = rd;
+    if (!lambert) ud = normalize(rd);
+    const bool ball = lambert || metal;       // scatters by a point in the unit ball
+    const bool given = preset && lambert;
+    float ratio = 1.0f, r0 = 0.0f, base = 1.0f, exponent = 0.33333f;
+    bool reflected = false;
+    if (glass) {
+        const float ior = mb.y;
+        ratio = g.front ? 1.0f / ior : ior;
+        const float cos_t = fminf(dot(neg(ud), normal), 1.0f);
+        const float sin_t = sqrtf(1.0f - cos_t * cos_t);
+        reflected = ratio * sin_t > 1.0f;
+        r0 = (1.0f - ratio) / (1.0f + ratio);
+        r0 = r0 * r0;
+        base = 1.0f - cos_t;
+        exponent = 5.0f;
+    } else if (!given) {
+        base = rng.f();
+    }
+    float power = 1.0f;
+    if (!given && !reflected) power = M::pow(base, exponent);
+    f3 dir;
+    if (ball) {
+        // in_unit_sphere: radius (1 where the direction is given), polar
+        // angle, azimuth
+        const float theta = 3.14159265358979f * (given ? pu_theta : rng.f());
+        const float phi = 2.0f * 3.14159265358979f * (given ? pu_phi : rng.f());
+        float st, ct, sp, cph;
+        M::sincos(theta, &st, &ct);
+        M::sincos(phi, &sp, &cph);
+        const f3 s = mk(power * st * cph, power * st * sp, power * ct);
+        if (lambert) {
+            dir = add(normal, normalize(s));
+            if (fabsf(dir.x) < 1e-8f && fabsf(dir.y) < 1e-8f && fabsf(dir.z) < 1e-8f) dir = normal;
         } else {
-            s = rng.in_unit_sphere<MATH>();
+            dir = add(reflect(ud, normal), scale(mb.x, s));
+            if (SEM == SEM_WGSL && !(dot(dir, normal) > 0.0f)) {
+                *color_io = mul(color, mk(0.0f, 0.0f, 0.0f));
+                return false;
+            }
         }
-        f3 dir = add(normal, normalize(s));
-        if (fabsf(dir.x) < 1e-8f && fabsf(dir.y) < 1e-8f && fabsf(dir.z) < 1e-8f) dir = normal;
-        f3 att = use_tex ? tex_sample(sc.textures[tex_id], hu, hv, SEM == SEM_WGSL) : mk(ma.x, ma.y, ma.z);
-        if (COUNT && use_tex) scn->textured++;
-        *ro_io = hp;
-        *rd_io = dir;
-        *color_io = mul(color, att);
-        return true;
+    } else {
+        if (!reflected) reflected = r0 + (1.0f - r0) * power > rng.f();
+        dir = reflected ? reflect(ud, normal) : refract(ud, normal, ratio);
     }
-    if (mtype == ORN_METAL) {
-        f3 dir = add(reflect(normalize(rd), normal), scale(mb.x, rng.in_unit_sphere<MATH>()));
-        f3 att = use_tex ? tex_sample(sc.textures[tex_id], hu, hv, SEM == SEM_WGSL) : mk(ma.x, ma.y, ma.z);
-        if (COUNT && use_tex) scn->textured++;
-        if (SEM == SEM_WGSL && !(dot(dir, normal) > 0.0f)) {
-            *color_io = mul(color, mk(0.0f, 0.0f, 0.0f));
-            return false;
-        }
-        *ro_io = hp;
-        *rd_io = dir;
-        *color_io = mul(color, att);
-        return true;
-    }
-    if (mtype == ORN_DIELECTRIC) {
-        float ior = mb.y;
-        float ratio = front ? 1.0f / ior : ior;
-        f3 ud = normalize(rd);
-        float cos_t = fminf(dot(neg(ud), normal), 1.0f);
-        float sin_t = sqrtf(1.0f - cos_t * cos_t);
-        bool refl = ratio * sin_t > 1.0f;
-        if (!refl) {
-            float r0 = (1.0f - ratio) / (1.0f + ratio);
-            r0 = r0 * r0;
-            float pr = r0 + (1.0f - r0) * M::pow(1.0f - cos_t, 5.0f);
-            refl = pr > rng.f();
-        }
-        f3 dir = refl ? reflect(ud, normal) : refract(ud, normal, ratio);
-        *ro_io = hp;
-        *rd_io = dir;
-        *color_io = mul(color, mk(1.0f, 1.0f, 1.0f));
-        return true;
-    }
-    f3 em = mk(0.0f, 0.0f, 0.0f);
-    if (mtype == ORN_DIFFUSE_LIGHT) {
-        em = use_tex ? tex_sample(sc.textures[tex_id], hu, hv, SEM == SEM_WGSL) : mk(ma.x, ma.y, ma.z);
-        if (COUNT && use_tex) scn->textured++;
-    }
-    *color_io = mul(color, em);
-    return false;
+    *ro_io = g.hp;
+    *rd_io = dir;
+    *color_io = mul(color, att);
+    return true;
 }
 
 template <int SEM, int MATH, bool COUNT>

@@ -31,6 +31,23 @@ constexpr int kSmemStack = ORN_SMEM_STACK;
 #endif
 constexpr int kMegaMinBlocks = ORN_MEGA_MIN_BLOCKS;
 
+// The same for the kernel on the near-first trees, and the node visits that a
+// lane makes per pass of its loop.
+#ifndef ORN_NEAR_MIN_BLOCKS
+#define ORN_NEAR_MIN_BLOCKS 5
+#endif
+constexpr int kNearMinBlocks = ORN_NEAR_MIN_BLOCKS;
+#ifndef ORN_NEAR_STEPS
+#define ORN_NEAR_STEPS 8
+#endif
+constexpr int kNearSteps = ORN_NEAR_STEPS;
+
+// Node visits of near_step (pt_near.cuh) between looks at triangles and shapes.
+#ifndef ORN_NEAR_INNER
+#define ORN_NEAR_INNER 4
+#endif
+constexpr int kNearInner = ORN_NEAR_INNER;
+
 // Radiance-cache side of a cached megakernel launch.  Every pixel traces one
 // sample, with next-event estimation: at a lambertian vertex whose scattered
 // ray will be traced, a point on an emissive mesh triangle is sampled by area

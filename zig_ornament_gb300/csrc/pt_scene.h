@@ -30,6 +30,10 @@ enum { MATH_PORTABLE = 0, MATH_DEVICE = 1 };  // transcendental implementation
 // ERR_MMA: a tensor-core wait timed out; ERR_WAIT: a wavefront queue wait timed out
 enum { ERR_STACK = 1u, ERR_VISITS = 2u, ERR_MMA = 4u, ERR_WAIT = 8u };
 constexpr uint32_t kRefIndexMask = 0x3FFFFFFFu;
+// Stack of the near-first traversal in words (two per entry; pt_near.cuh), and
+// the mark on a triangle id whose leaf box in its trees is not its own.
+constexpr int kNearStackWords = 128;
+constexpr uint32_t kNearOwnBox = 0x80000000u;
 
 struct TexDesc {
     const unsigned char* data;
@@ -51,6 +55,12 @@ struct SceneDev {
     const TexDesc* textures;
     uint32_t textures_len;
     uint32_t watertight;        // 1: watertight triangle test (orn_state.triangle_test), 0: the reference's
+    // Other trees over the same primitives (tree_build.cu), for the traversal
+    // of pt_near.cuh: behind the nodes above in the same array and format.
+    // `near` is 0 when the scene's arrays do not have what its proof of equal
+    // results needs; the nodes above are then walked everywhere.
+    uint32_t near;
+    uint32_t nroot;             // reference of the TLAS root
 };
 
 }  // namespace orn

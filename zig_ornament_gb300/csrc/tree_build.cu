@@ -1,0 +1,721 @@
+// tree_build.cu — the device side of scene creation: the kernels' node array,
+// and the trees that pt_near.cuh traverses.
+//
+//   1. The blob's nodes go to the device as they are; one pass writes the
+//      kernels' node array (pt_scene.h), a second finds every node's parent
+//      and checks what the near-first traversal's proof of equal results
+//      needs: each stored box holds the boxes stored below it, a triangle's
+//      box is that of its vertices, no node has two parents, and no walk can
+//      need more than the reference's 64 stack entries.  A blob without one
+//      of these (other builders' padding, shared subtrees) keeps the
+//      reference's walk.
+//   2. Every triangle finds the mesh it belongs to by its parents; triangles
+//      and TLAS leaves are sorted by (tree, Morton code of the box centre).
+//   3. Binary trees by parallel locally-ordered clustering (Meister and
+//      Bittner, "Parallel Locally-Ordered Clustering for Bounding Volume
+//      Hierarchy Construction", TVCG 2018), all meshes and the TLAS in the
+//      same passes: each cluster picks the neighbour within kRadius places of
+//      the same tree whose union box has the least area; pairs that pick each
+//      other merge.
+//   4. Nodes written top-down in treelets: a thread opens the largest inner
+//      node of its treelet until it has eight below it, and the nodes inside
+//      and the eight below are stored next to each other.
+//
+// Results do not depend on these trees, only speed does.
+#include <cub/device/device_radix_sort.cuh>
+#include <cub/device/device_select.cuh>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "tree_build.h"
+
+namespace orn {
+namespace {
+
+constexpr uint32_t kNone = 0xffffffffu;
+constexpr uint32_t kTlasTree = 0x3fffffffu;   // tree id of the TLAS (meshes: their root's BLAS index)
+constexpr uint32_t kDepthLimit = 64;          // the reference's stack entries
+constexpr int kRadius = 16;
+constexpr int kNnBlock = 256;
+constexpr uint32_t kMostSlivers = 64;
+constexpr float kSliver = 1024.0f;
+constexpr uint32_t kNearDepthLimit = kNearStackWords / 2;   // levels of TLAS and BLAS together (one entry of two words each)
+
+// Counters and flags of one build (device; read back between phases).
+struct State {
+    uint32_t bad;         // the blob lacks something the near-first traversal needs
+    uint32_t huge;
+    uint32_t slivers;
+    uint32_t prims;       // triangles that belong to a mesh, and reachable TLAS leaves
+    uint32_t trees;       // meshes with triangles, and the TLAS
+    uint32_t blas_depth, tlas_depth;
+    uint32_t next_node;   // binary inner nodes made
+    uint32_t written;     // nodes placed
+    uint32_t meshes;      // mesh leaves among them
+    uint32_t queue[2];    // treelets to write, this level and the next
+    uint32_t selected;
+    uint32_t near_depth[2];   // levels of the deepest BLAS, and of the TLAS
+    uint32_t root;        // reference of the TLAS root
+};
+
+__device__ __forceinline__ uint32_t ref_of(const orn_bvh_node* nodes, uint32_t i, uint32_t offset) {
+    return (offset + i) | (nodes[i].node_type << 30);
+}
+
+// The kernels' node array.  A triangle keeps its vertices as given, so
+// triangles sharing an edge see the same floats (the watertight test relies
+// on it), and the two edges the reference's test subtracts on the fly
+// (bvh.hip.h:81-82) — the same single-precision subtractions.
+__global__ void relayout_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t T,
+                                const orn_bvh_node* __restrict__ blas, uint32_t B, const float4* __restrict__ xforms,
+                                float4* __restrict__ out, State* st) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= T + B) return;
+    const bool top = i < T;
+    const orn_bvh_node n = top ? tlas[i] : blas[i - T];
+    const float* a = n.left_aabb_min_or_v0;
+    const float* b = n.left_aabb_max_or_v1;
+    const float* c = n.right_aabb_min_or_v2;
+    const float* e = n.right_aabb_max_or_v3;
+    float4* o = out + (size_t)i * 4;
+    if (n.node_type == ORN_NODE_INTERNAL) {
+        const orn_bvh_node* src = top ? tlas : blas;
+        const uint32_t off = top ? 0u : T;
+        o[0] = make_float4(a[0], a[1], a[2], __uint_as_float(ref_of(src, n.left_or_custom_id, off)));
+        o[1] = make_float4(b[0], b[1], b[2], __uint_as_float(ref_of(src, n.right_or_material_index, off)));
+        o[2] = make_float4(c[0], c[1], c[2], __uint_as_float(ORN_NODE_INTERNAL));
+        o[3] = make_float4(e[0], e[1], e[2], 0.0f);
+        bool ok = true;
+        for (int k = 0; k < 3; ++k)
+            ok = ok && fabsf(a[k]) < 1e30f && fabsf(b[k]) < 1e30f && fabsf(c[k]) < 1e30f && fabsf(e[k]) < 1e30f;
+        if (!ok) st->huge = 1u;
+    } else if (n.node_type == ORN_NODE_TRIANGLE) {
+        o[0] = make_float4(a[0], a[1], a[2], __uint_as_float(n.left_or_custom_id));
+        o[1] = make_float4(b[0], b[1], b[2], c[0] - a[0]);
+        o[2] = make_float4(c[0], c[1], c[2], c[1] - a[1]);
+        o[3] = make_float4(b[0] - a[0], b[1] - a[1], b[2] - a[2], c[2] - a[2]);
+    } else {   // sphere / mesh leaf: inverse rows 0..2 inline
+        const float4* m = xforms + (size_t)n.transform_id * 2 * 4;
+        const float4 r0 = m[0], r1 = m[1], r2 = m[2];
+        const uint32_t root = n.node_type == ORN_NODE_MESH ? ref_of(blas, n.left_or_custom_id, T) : 0u;
+        o[0] = r0;
+        o[1] = r1;
+        o[2] = make_float4(r2.x, r2.y, r2.z, __uint_as_float(n.node_type));
+        o[3] = make_float4(r2.w, __uint_as_float(n.right_or_material_index), __uint_as_float(n.transform_id),
+                           __uint_as_float(root));
+    }
+}
+
+__device__ __forceinline__ void stored_box(const orn_bvh_node& n, bool right, float* lo, float* hi) {
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = right ? n.right_aabb_min_or_v2[k] : n.left_aabb_min_or_v0[k];
+        hi[k] = right ? n.right_aabb_max_or_v3[k] : n.left_aabb_max_or_v1[k];
+    }
+}
+__device__ __forceinline__ void triangle_box(const orn_bvh_node& n, float* lo, float* hi) {
+    for (int k = 0; k < 3; ++k) {
+        const float a = n.left_aabb_min_or_v0[k], b = n.left_aabb_max_or_v1[k], c = n.right_aabb_min_or_v2[k];
+        lo[k] = fminf(fminf(a, b), c);
+        hi[k] = fmaxf(fmaxf(a, b), c);
+    }
+}
+
+// Parents (bit 31: the right child) of the children of nodes[0..n), and the
+// checks on their boxes.
+__global__ void parents_kernel(const orn_bvh_node* __restrict__ nodes, uint32_t n, uint32_t* __restrict__ parent,
+                               State* st) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const orn_bvh_node nd = nodes[i];
+    if (nd.node_type != ORN_NODE_INTERNAL) return;
+    bool ok = true;
+    for (int side = 0; side < 2; ++side) {
+        const uint32_t c = side ? nd.right_or_material_index : nd.left_or_custom_id;
+        if (atomicExch(&parent[c], i | (side ? 0x80000000u : 0u)) != kNone) ok = false;
+        float lo[3], hi[3];
+        stored_box(nd, side != 0, lo, hi);
+        const orn_bvh_node ch = nodes[c];
+        if (ch.node_type == ORN_NODE_INTERNAL) {
+            for (int s2 = 0; s2 < 2; ++s2) {
+                float clo[3], chi[3];
+                stored_box(ch, s2 != 0, clo, chi);
+                for (int k = 0; k < 3; ++k) ok = ok && clo[k] >= lo[k] && chi[k] <= hi[k];
+            }
+        } else if (ch.node_type == ORN_NODE_TRIANGLE) {
+            float tlo[3], thi[3];
+            triangle_box(ch, tlo, thi);
+            for (int k = 0; k < 3; ++k) ok = ok && tlo[k] == lo[k] && thi[k] == hi[k];
+        }
+    }
+    if (!ok) st->bad = 1u;
+}
+
+__global__ void roots_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t T, uint8_t* __restrict__ is_root) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < T && tlas[i].node_type == ORN_NODE_MESH) is_root[tlas[i].left_or_custom_id] = 1;
+}
+
+__device__ __forceinline__ uint32_t spread3(uint32_t v) {   // 10 bits to every third bit
+    v = (v | (v << 16)) & 0x030000ffu;
+    v = (v | (v << 8)) & 0x0300f00fu;
+    v = (v | (v << 4)) & 0x030c30c3u;
+    return (v | (v << 2)) & 0x09249249u;
+}
+__device__ __forceinline__ uint32_t morton30(const float* lo, const float* hi, const float* tlo, const float* thi) {
+    uint32_t code = 0;
+    for (int k = 0; k < 3; ++k) {
+        const float ext = thi[k] - tlo[k];
+        const float x = ext > 0.0f ? (0.5f * lo[k] + 0.5f * hi[k] - tlo[k]) / ext : 0.0f;
+        code |= spread3((uint32_t)fminf(fmaxf(x * 1024.0f, 0.0f), 1023.0f)) << k;
+    }
+    return code;
+}
+
+// A triangle whose edges are so nearly parallel that its hit test can be off
+// by far more than its distance to its box.
+__device__ __forceinline__ bool is_sliver(const orn_bvh_node& n) {
+    float e1[3], e2[3];
+    for (int k = 0; k < 3; ++k) {
+        e1[k] = n.left_aabb_max_or_v1[k] - n.left_aabb_min_or_v0[k];
+        e2[k] = n.right_aabb_min_or_v2[k] - n.left_aabb_min_or_v0[k];
+    }
+    const float cx = e1[1] * e2[2] - e1[2] * e2[1], cy = e1[2] * e2[0] - e1[0] * e2[2], cz = e1[0] * e2[1] - e1[1] * e2[0];
+    const float area = sqrtf(cx * cx + cy * cy + cz * cz);
+    const float l1 = sqrtf(e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2]);
+    const float l2 = sqrtf(e2[0] * e2[0] + e2[1] * e2[1] + e2[2] * e2[2]);
+    return l1 * l2 > 0.0f && !(area * kSliver > l1 * l2);   // (a zero edge gives det = 0: never a hit)
+}
+
+// Sort key and box of every primitive, by node index (BLAS, then TLAS).
+__global__ void prims_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t T, const orn_bvh_node* __restrict__ blas,
+                             uint32_t B, const uint32_t* __restrict__ bparent, const uint32_t* __restrict__ tparent,
+                             const uint8_t* __restrict__ is_root, unsigned long long* __restrict__ keys,
+                             uint32_t* __restrict__ vals, float4* __restrict__ boxes, uint8_t* __restrict__ tree_used,
+                             State* st) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= B + T) return;
+    keys[i] = 1ull << 60;   // after every tree: not a primitive of one
+    vals[i] = i;
+    const bool top = i >= B;
+    const uint32_t self = top ? i - B : i;
+    const orn_bvh_node nd = top ? tlas[self] : blas[self];
+    if (nd.node_type == ORN_NODE_INTERNAL) return;
+    float lo[3], hi[3], tlo[3], thi[3];
+    uint32_t tree = kNone;
+    uint32_t depth = 0;
+    const uint32_t* parent = top ? tparent : bparent;
+    uint32_t cur = self;
+    for (;;) {   // up to the top: the tree is the one marked root on the way
+        if (top ? cur == T - 1 : is_root[cur] != 0) {
+            if (tree != kNone) st->bad = 1u;   // a mesh inside another
+            tree = top ? kTlasTree : cur;
+        }
+        const uint32_t p = parent[cur];
+        if (p == kNone) break;
+        cur = p & 0x7fffffffu;
+        if (tree == kNone) ++depth;
+        if (depth > kDepthLimit) {
+            st->bad = 1u;
+            return;
+        }
+    }
+    if (tree == kNone) return;   // not reachable from any shape
+    uint32_t* deepest = top ? &st->tlas_depth : &st->blas_depth;
+    if (depth > *(volatile uint32_t*)deepest) atomicMax(deepest, depth);
+    const uint32_t p = parent[self];
+    if (top) {
+        if (self != T - 1) {
+            stored_box(tlas[p & 0x7fffffffu], (p >> 31) != 0, lo, hi);
+        } else {
+            for (int k = 0; k < 3; ++k) {   // the only shape: its own node carries its box
+                lo[k] = nd.left_aabb_min_or_v0[k];
+                hi[k] = nd.left_aabb_max_or_v1[k];
+            }
+        }
+        float ext = 0.0f;
+        for (int k = 0; k < 3; ++k) ext = fmaxf(ext, fmaxf(fabsf(lo[k]), fabsf(hi[k])));
+        if (!(ext < 1e30f)) st->bad = 1u;
+        const orn_bvh_node root = tlas[T - 1];
+        if (T > 1) {
+            float l2[3], h2[3];
+            stored_box(root, false, tlo, thi);
+            stored_box(root, true, l2, h2);
+            for (int k = 0; k < 3; ++k) {
+                tlo[k] = fminf(tlo[k], l2[k]);
+                thi[k] = fmaxf(thi[k], h2[k]);
+            }
+        } else {
+            for (int k = 0; k < 3; ++k) {
+                tlo[k] = lo[k];
+                thi[k] = hi[k];
+            }
+        }
+    } else {
+        triangle_box(nd, lo, hi);
+        const orn_bvh_node root = blas[tree];
+        if (root.node_type == ORN_NODE_INTERNAL) {
+            float l2[3], h2[3];
+            stored_box(root, false, tlo, thi);
+            stored_box(root, true, l2, h2);
+            for (int k = 0; k < 3; ++k) {
+                tlo[k] = fminf(tlo[k], l2[k]);
+                thi[k] = fmaxf(thi[k], h2[k]);
+            }
+        } else {
+            for (int k = 0; k < 3; ++k) {
+                tlo[k] = lo[k];
+                thi[k] = hi[k];
+            }
+        }
+        bool finite = true;
+        for (int k = 0; k < 3; ++k) finite = finite && fabsf(lo[k]) < 1e30f && fabsf(hi[k]) < 1e30f;
+        if (!finite) st->bad = 1u;
+    }
+    keys[i] = ((unsigned long long)tree << 30) | morton30(lo, hi, tlo, thi);
+    float own_box = 0.0f;   // a mark: the box given here is not the triangle's own
+    if (!top && tree != self && is_sliver(nd)) {   // visited wherever its mesh is
+        atomicAdd(&st->slivers, 1u);
+        own_box = __uint_as_float(1u);
+        for (int k = 0; k < 3; ++k) {
+            lo[k] = tlo[k];
+            hi[k] = thi[k];
+        }
+    }
+    boxes[2 * (size_t)i] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+    boxes[2 * (size_t)i + 1] = make_float4(hi[0], hi[1], hi[2], own_box);
+    atomicAdd(&st->prims, 1u);
+    uint8_t* used = top ? tree_used + B : tree_used + tree;
+    if (*used == 0) *used = 1;
+}
+
+__global__ void count_trees_kernel(const uint8_t* __restrict__ used, uint32_t n, State* st) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned m = __ballot_sync(0xffffffffu, i < n && used[i] != 0);
+    if ((threadIdx.x & 31u) == 0 && m) atomicAdd(&st->trees, (uint32_t)__popc(m));
+}
+
+// ---- binary trees ------------------------------------------------------------------------------
+// Node k < n is the k-th primitive in sorted order; inner nodes follow.
+// node_box[2k], [2k+1]: corners, the tree id in the first one's w.
+__global__ void leaves_kernel(const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ vals,
+                              const float4* __restrict__ boxes, uint32_t n, float4* __restrict__ node_box,
+                              uint32_t* __restrict__ cluster) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const uint32_t v = vals[k];
+    float4 lo = boxes[2 * (size_t)v];
+    lo.w = __uint_as_float((uint32_t)(keys[k] >> 30));
+    node_box[2 * (size_t)k] = lo;
+    node_box[2 * (size_t)k + 1] = boxes[2 * (size_t)v + 1];
+    cluster[k] = k;
+}
+
+__device__ __forceinline__ float half_area(float4 lo, float4 hi) {
+    const float x = hi.x - lo.x, y = hi.y - lo.y, z = hi.z - lo.z;
+    return x * y + y * z + z * x;
+}
+__device__ __forceinline__ float4 min4(float4 a, float4 b) {
+    return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), a.w);
+}
+__device__ __forceinline__ float4 max4(float4 a, float4 b) {
+    return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), a.w);
+}
+
+// Each cluster's choice among its neighbours.  Pairs are ordered by (area,
+// i xor j): the least pair of a tree is chosen from both sides, so every
+// round merges something, and among equal boxes each index has another
+// partner.
+__global__ void __launch_bounds__(kNnBlock)
+neighbour_kernel(const uint32_t* __restrict__ cluster, uint32_t m, const float4* __restrict__ node_box,
+                 uint32_t* __restrict__ nn) {
+    __shared__ float4 slo[kNnBlock + 2 * kRadius], shi[kNnBlock + 2 * kRadius];
+    const int first = (int)(blockIdx.x * kNnBlock) - kRadius;
+    for (int t = threadIdx.x; t < kNnBlock + 2 * kRadius; t += kNnBlock) {
+        const int g = first + t;
+        float4 lo = make_float4(0, 0, 0, __uint_as_float(kNone)), hi = lo;
+        if (g >= 0 && g < (int)m) {
+            const uint32_t c = cluster[g];
+            lo = node_box[2 * (size_t)c];
+            hi = node_box[2 * (size_t)c + 1];
+        }
+        slo[t] = lo;
+        shi[t] = hi;
+    }
+    __syncthreads();
+    const uint32_t i = blockIdx.x * kNnBlock + threadIdx.x;
+    if (i >= m) return;
+    const int self = threadIdx.x + kRadius;
+    const float4 lo = slo[self], hi = shi[self];
+    const uint32_t tree = __float_as_uint(lo.w);
+    uint32_t best = kNone;
+    float area = 0.0f;
+    for (int r = -kRadius; r <= kRadius; ++r) {
+        if (r == 0 || __float_as_uint(slo[self + r].w) != tree) continue;
+        const float a = half_area(min4(lo, slo[self + r]), max4(hi, shi[self + r]));
+        const uint32_t j = i + r;
+        if (best == kNone || a < area || (a == area && (i ^ j) < (i ^ best))) {
+            best = j;
+            area = a;
+        }
+    }
+    nn[i] = best;
+}
+
+// For trees that merge too slowly: neighbours in pairs, from an even or odd place.
+__global__ void pair_kernel(const uint32_t* __restrict__ cluster, uint32_t m, const float4* __restrict__ node_box,
+                            uint32_t odd, uint32_t* __restrict__ nn) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const uint32_t j = ((i + odd) & 1u) ? i - 1u : i + 1u;
+    nn[i] = j < m && __float_as_uint(node_box[2 * (size_t)cluster[i]].w) ==
+                         __float_as_uint(node_box[2 * (size_t)cluster[j]].w) ? j : kNone;
+}
+
+__global__ void merge_kernel(uint32_t* __restrict__ cluster, uint32_t m, const uint32_t* __restrict__ nn, uint32_t n,
+                             float4* __restrict__ node_box, uint2* __restrict__ child, uint8_t* __restrict__ keep,
+                             State* st) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const uint32_t j = nn[i];
+    const bool pair = j != kNone && nn[j] == i;
+    keep[i] = !pair || i < j;
+    if (!pair || i > j) return;
+    const uint32_t a = cluster[i], b = cluster[j];
+    const uint32_t id = n + atomicAdd(&st->next_node, 1u);
+    node_box[2 * (size_t)id] = min4(node_box[2 * (size_t)a], node_box[2 * (size_t)b]);
+    node_box[2 * (size_t)id + 1] = max4(node_box[2 * (size_t)a + 1], node_box[2 * (size_t)b + 1]);
+    child[id - n] = make_uint2(a, b);
+    cluster[i] = id;
+}
+
+// ---- the node array ----------------------------------------------------------------------------
+struct Work {   // a treelet to write: its root, that node's place, and the levels above it
+    uint32_t node, place, depth;
+};
+
+// What the writing kernels share.
+struct Emit {
+    uint32_t n, B, T;
+    const float4* node_box;
+    const uint2* child;
+    const uint32_t* vals;      // primitive k's node index in the blob (BLAS, then TLAS)
+    const float4* nodes;       // the kernels' node array (TLAS, then BLAS)
+    float4* out;               // the same array: the new nodes go behind
+    uint32_t first;            // index of the first new node
+    uint32_t* root_of;         // by BLAS node index: the reference of a mesh's root
+    uint32_t* mesh_place;      // places of the mesh leaves
+    State* st;
+};
+
+__device__ __forceinline__ float half_area_of(const Emit& e, uint32_t c) {
+    return half_area(e.node_box[2 * (size_t)c], e.node_box[2 * (size_t)c + 1]);
+}
+// Reference to tree node c stored at `place`.
+__device__ __forceinline__ uint32_t place_ref(const Emit& e, uint32_t c, uint32_t place) {
+    place += e.first;
+    if (c >= e.n) return place;   // ORN_NODE_INTERNAL == 0
+    const uint32_t v = e.vals[c];
+    if (v < e.B) return place | ((uint32_t)ORN_NODE_TRIANGLE << 30);
+    const bool sphere = __float_as_uint(e.nodes[(size_t)(v - e.B) * 4 + 2].w) == ORN_NODE_SPHERE;
+    return place | ((uint32_t)(sphere ? ORN_NODE_SPHERE : ORN_NODE_MESH) << 30);
+}
+__device__ __forceinline__ void write_primitive(const Emit& e, uint32_t c, uint32_t place) {
+    const uint32_t v = e.vals[c];
+    const float4* src = e.nodes + 4 * (size_t)(v < e.B ? e.T + v : v - e.B);
+    float4 a = src[0];
+    const float4 mid = src[2];
+    if (v < e.B && __float_as_uint(e.node_box[2 * (size_t)c + 1].w) != 0u)
+        a.w = __uint_as_float(__float_as_uint(a.w) | kNearOwnBox);
+    e.out[4 * (size_t)place] = a;
+    e.out[4 * (size_t)place + 1] = src[1];
+    e.out[4 * (size_t)place + 2] = mid;
+    e.out[4 * (size_t)place + 3] = src[3];
+    if (v >= e.B && __float_as_uint(mid.w) == ORN_NODE_MESH) e.mesh_place[atomicAdd(&e.st->meshes, 1u)] = place;
+}
+
+// One cluster per tree is left: its root.
+__global__ void seed_kernel(Emit e, const uint32_t* __restrict__ cluster, uint32_t trees, Work* __restrict__ queue) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= trees) return;
+    const uint32_t c = cluster[i];
+    const uint32_t tree = __float_as_uint(e.node_box[2 * (size_t)c].w);
+    const uint32_t place = atomicAdd(&e.st->written, 1u);
+    if (c < e.n) write_primitive(e, c, place);
+    else queue[atomicAdd(&e.st->queue[0], 1u)] = Work{c, place, 0u};
+    if (tree == kTlasTree) e.st->root = place_ref(e, c, place);
+    else e.root_of[tree] = place_ref(e, c, place);
+}
+
+__global__ void __launch_bounds__(128)
+treelet_kernel(Emit e, const Work* __restrict__ queue, uint32_t count, Work* __restrict__ next, int next_slot) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= count) return;
+    const Work work = queue[t];
+    // inner[i]: opened nodes, the root first; below: the nodes under them,
+    // each with the opened node and side it hangs from
+    uint32_t inner[7], place[7], depth[7], below[8], hang[8];
+    int ni = 1, nb = 2;
+    inner[0] = work.node;
+    place[0] = work.place;
+    depth[0] = work.depth;
+    for (int side = 0; side < 2; ++side) {
+        below[side] = side ? e.child[work.node - e.n].y : e.child[work.node - e.n].x;
+        hang[side] = (uint32_t)side;
+    }
+    // opened children: which opened node hangs from (inner, side)
+    int opened[14];
+    for (int k = 0; k < 14; ++k) opened[k] = -1;
+    while (nb < 8) {
+        int open = -1;
+        float area = -1.0f;
+        for (int k = 0; k < nb; ++k) {
+            if (below[k] < e.n) continue;
+            const float a = half_area_of(e, below[k]);
+            if (a > area) {
+                area = a;
+                open = k;
+            }
+        }
+        if (open < 0) break;
+        const uint32_t c = below[open];
+        inner[ni] = c;
+        depth[ni] = depth[hang[open] >> 1] + 1u;
+        opened[hang[open]] = ni;
+        below[open] = e.child[c - e.n].x;
+        below[nb] = e.child[c - e.n].y;
+        hang[open] = (uint32_t)(2 * ni);
+        hang[nb] = (uint32_t)(2 * ni + 1);
+        ++ni;
+        ++nb;
+    }
+    uint32_t at = atomicAdd(&e.st->written, (uint32_t)(ni - 1 + nb));
+    for (int k = 1; k < ni; ++k) place[k] = at++;
+    uint32_t refs[14];
+    uint32_t more = 0;
+    for (int k = 0; k < 14; ++k)
+        if (opened[k] >= 0) refs[k] = e.first + place[opened[k]];
+    for (int k = 0; k < nb; ++k) {
+        refs[hang[k]] = place_ref(e, below[k], at + (uint32_t)k);
+        if (below[k] < e.n) write_primitive(e, below[k], at + (uint32_t)k);
+        else ++more;
+    }
+    uint32_t q = more ? atomicAdd(&e.st->queue[next_slot], more) : 0u;
+    uint32_t deepest = 0;
+    for (int k = 0; k < nb; ++k) {
+        const uint32_t d = depth[hang[k] >> 1] + 1u;
+        deepest = max(deepest, d);
+        if (below[k] >= e.n) next[q++] = Work{below[k], at + (uint32_t)k, d};
+    }
+    const bool top = __float_as_uint(e.node_box[2 * (size_t)work.node].w) == kTlasTree;
+    if (deepest > *(volatile uint32_t*)&e.st->near_depth[top]) atomicMax(&e.st->near_depth[top], deepest);
+    for (int k = 0; k < ni; ++k) {
+        const uint2 ch = e.child[inner[k] - e.n];
+        float4 llo = e.node_box[2 * (size_t)ch.x], lhi = e.node_box[2 * (size_t)ch.x + 1];
+        float4 rlo = e.node_box[2 * (size_t)ch.y], rhi = e.node_box[2 * (size_t)ch.y + 1];
+        llo.w = __uint_as_float(refs[2 * k]);
+        lhi.w = __uint_as_float(refs[2 * k + 1]);
+        rlo.w = __uint_as_float(ORN_NODE_INTERNAL);
+        rhi.w = 0.0f;
+        float4* o = e.out + 4 * (size_t)place[k];
+        o[0] = llo;
+        o[1] = lhi;
+        o[2] = rlo;
+        o[3] = rhi;
+    }
+}
+
+// Points the mesh leaves of the written array at their new roots.
+__global__ void meshes_kernel(float4* __restrict__ out, uint32_t T, const uint32_t* __restrict__ root_of,
+                              const uint32_t* __restrict__ mesh_place, uint32_t meshes) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= meshes) return;
+    float4* o = out + 4 * (size_t)mesh_place[i];
+    const uint32_t old = __float_as_uint(o[3].w) & kRefIndexMask;   // in the kernels' array: T + BLAS index
+    o[3].w = __uint_as_float(root_of[old - T]);
+}
+
+inline unsigned blocks(size_t n, unsigned per) { return (unsigned)((n + per - 1) / per); }
+
+// A bump allocator over one device allocation.
+struct Arena {
+    unsigned char* base = nullptr;
+    size_t used = 0, size = 0;
+    template <class T>
+    T* take(size_t count) {
+        used = (used + 255) & ~(size_t)255;
+        T* p = (T*)(base + used);
+        used += count * sizeof(T);
+        return p;
+    }
+};
+
+#define WB(call)                               \
+    do {                                       \
+        const cudaError_t e_ = (call);         \
+        if (e_ != cudaSuccess) return e_;      \
+    } while (0)
+
+struct Build {
+    const orn_scene_blob* blob;
+    const float4* xforms;
+    SceneDev* scene;
+    std::vector<void*>* allocs;
+    cudaStream_t s;
+    State* d_state = nullptr;
+    State h{};
+    orn_bvh_node *tlas = nullptr, *blas = nullptr;
+    float4* nodes = nullptr;
+    void* second = nullptr;   // the second phase's arena
+
+    cudaError_t read_state() {
+        WB(cudaMemcpyAsync(&h, d_state, sizeof(State), cudaMemcpyDeviceToHost, s));
+        return cudaStreamSynchronize(s);
+    }
+    cudaError_t near_trees(Arena& a);
+};
+
+// Bytes of the first phase's arrays (all nodes), and of the second's (n primitives).
+size_t first_bytes(size_t T, size_t B) { return 64 * (T + B) + 4 * (T + B) + 2 * (B + 1) + 24 * (T + B) + 32 * (T + B) + 32 * 256; }
+size_t second_bytes(size_t n, size_t T, size_t B, size_t temp) {
+    return temp + 64 * n + 8 * n + 13 * n + 24 * n + 4 * (T + B) + 32 * 256;
+}
+
+cudaError_t Build::near_trees(Arena& a) {
+    const uint32_t T = blob->tlas_nodes_len, B = blob->blas_nodes_len, N = T + B;
+    uint32_t* bparent = a.take<uint32_t>(B);
+    uint32_t* tparent = a.take<uint32_t>(T);
+    uint8_t* is_root = a.take<uint8_t>((size_t)B + 1);
+    uint8_t* used = a.take<uint8_t>((size_t)B + 1);
+    WB(cudaMemsetAsync(bparent, 0xff, (size_t)B * 4, s));
+    WB(cudaMemsetAsync(tparent, 0xff, (size_t)T * 4, s));
+    WB(cudaMemsetAsync(is_root, 0, (size_t)B + 1, s));
+    WB(cudaMemsetAsync(used, 0, (size_t)B + 1, s));
+    parents_kernel<<<blocks(T, 256), 256, 0, s>>>(tlas, T, tparent, d_state);
+    if (B) parents_kernel<<<blocks(B, 256), 256, 0, s>>>(blas, B, bparent, d_state);
+    if (B) roots_kernel<<<blocks(T, 256), 256, 0, s>>>(tlas, T, is_root);
+    unsigned long long* keys = a.take<unsigned long long>(N);
+    unsigned long long* keys2 = a.take<unsigned long long>(N);
+    uint32_t* vals = a.take<uint32_t>(N);
+    uint32_t* vals2 = a.take<uint32_t>(N);
+    float4* boxes = a.take<float4>(2 * (size_t)N);
+    prims_kernel<<<blocks(N, 256), 256, 0, s>>>(tlas, T, blas, B, bparent, tparent, is_root, keys, vals, boxes, used,
+                                                d_state);
+    count_trees_kernel<<<blocks((size_t)B + 1, 256), 256, 0, s>>>(used, B + 1, d_state);
+    WB(cudaGetLastError());
+    WB(read_state());
+    const uint32_t n = h.prims, trees = h.trees;
+    if (h.bad || h.huge || h.slivers > kMostSlivers || h.tlas_depth + h.blas_depth > kDepthLimit || n == 0 ||
+        2 * (uint64_t)N > kRefIndexMask)
+        return cudaSuccess;
+    size_t sort_bytes = 0, select_bytes = 0;
+    WB(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys, keys2, vals, vals2, (int)N, 0, 61, s));
+    WB(cub::DeviceSelect::Flagged(nullptr, select_bytes, vals, is_root, vals2, &d_state->selected, (int)n, s));
+    const size_t temp_bytes = std::max(sort_bytes, select_bytes);
+    Arena a2;
+    a2.size = second_bytes(n, T, B, temp_bytes);
+    WB(cudaMalloc((void**)&a2.base, a2.size));
+    second = a2.base;
+    void* temp = a2.take<unsigned char>(temp_bytes);
+    size_t tb = sort_bytes;
+    WB(cub::DeviceRadixSort::SortPairs(temp, tb, keys, keys2, vals, vals2, (int)N, 0, 61, s));
+    float4* node_box = a2.take<float4>(4 * (size_t)n);
+    uint2* child = a2.take<uint2>(n);
+    uint32_t* cluster = a2.take<uint32_t>(n);
+    uint32_t* cluster2 = a2.take<uint32_t>(n);
+    uint32_t* nn = a2.take<uint32_t>(n);
+    uint8_t* keep_flag = a2.take<uint8_t>(n);
+    leaves_kernel<<<blocks(n, 256), 256, 0, s>>>(keys2, vals2, boxes, n, node_box, cluster);
+    WB(cudaGetLastError());
+    uint32_t m = n;
+    for (uint32_t round = 0; m > trees; ++round) {
+        if (round < 64) neighbour_kernel<<<blocks(m, kNnBlock), kNnBlock, 0, s>>>(cluster, m, node_box, nn);
+        else pair_kernel<<<blocks(m, 256), 256, 0, s>>>(cluster, m, node_box, round & 1u, nn);
+        merge_kernel<<<blocks(m, 256), 256, 0, s>>>(cluster, m, nn, n, node_box, child, keep_flag, d_state);
+        WB(cudaGetLastError());
+        size_t sb = select_bytes;
+        WB(cub::DeviceSelect::Flagged(temp, sb, cluster, keep_flag, cluster2, &d_state->selected, (int)m, s));
+        std::swap(cluster, cluster2);
+        WB(read_state());
+        m = h.selected;
+    }
+    Work* q0 = a2.take<Work>(n);
+    Work* q1 = a2.take<Work>(n);
+    Emit e;
+    e.n = n;
+    e.B = B;
+    e.T = T;
+    e.node_box = node_box;
+    e.child = child;
+    e.vals = vals2;
+    e.nodes = nodes;
+    e.root_of = a2.take<uint32_t>(B);
+    e.mesh_place = a2.take<uint32_t>(T);
+    e.st = d_state;
+    // a binary tree of k leaves has 2k - 1 nodes here as in the blob: the new
+    // ones are no more than those (build_scene_trees makes room for them)
+    e.first = N;
+    e.out = nodes + 4 * (size_t)N;
+    seed_kernel<<<blocks(trees, 128), 128, 0, s>>>(e, cluster, trees, q0);
+    WB(cudaGetLastError());
+    WB(read_state());
+    uint32_t level = 0;
+    for (uint32_t count = h.queue[0]; count; ++level) {
+        const int nx = (level & 1u) ? 0 : 1;
+        WB(cudaMemsetAsync(&d_state->queue[nx], 0, 4, s));
+        treelet_kernel<<<blocks(count, 128), 128, 0, s>>>(e, nx ? q0 : q1, count, nx ? q1 : q0, nx);
+        WB(cudaGetLastError());
+        WB(read_state());
+        count = h.queue[nx];
+    }
+    if (h.near_depth[0] + h.near_depth[1] > kNearDepthLimit) return cudaSuccess;
+    if (h.meshes) meshes_kernel<<<blocks(h.meshes, 128), 128, 0, s>>>(e.out, T, e.root_of, e.mesh_place, h.meshes);
+    WB(cudaGetLastError());
+    scene->nroot = h.root;
+    scene->near = 1u;
+    return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t build_scene_trees(const orn_scene_blob* blob, const float4* d_xforms, SceneDev* scene, NodeFacts* facts,
+                              std::vector<void*>* allocs, cudaStream_t s) {
+    const uint32_t T = blob->tlas_nodes_len, B = blob->blas_nodes_len;
+    Build b;
+    b.blob = blob;
+    b.xforms = d_xforms;
+    b.scene = scene;
+    b.allocs = allocs;
+    b.s = s;
+    void* nodes = nullptr;
+    WB(cudaMalloc(&nodes, 2 * ((size_t)T + B) * 64));
+    allocs->push_back(nodes);
+    b.nodes = (float4*)nodes;
+    scene->nodes = b.nodes;
+    scene->near = 0u;
+    Arena a;
+    a.size = first_bytes(T, B);
+    WB(cudaMalloc((void**)&a.base, a.size));
+    const cudaError_t e = [&]() -> cudaError_t {
+        // the transforms came through the default stream, which `s` does not wait for
+        WB(cudaStreamSynchronize(nullptr));
+        b.d_state = a.take<State>(1);
+        b.tlas = a.take<orn_bvh_node>(T);
+        b.blas = a.take<orn_bvh_node>(B);
+        WB(cudaMemsetAsync(b.d_state, 0, sizeof(State), s));
+        WB(cudaMemcpyAsync(b.tlas, blob->tlas_nodes, (size_t)T * 64, cudaMemcpyHostToDevice, s));
+        if (B) WB(cudaMemcpyAsync(b.blas, blob->blas_nodes, (size_t)B * 64, cudaMemcpyHostToDevice, s));
+        relayout_kernel<<<blocks((size_t)T + B, 256), 256, 0, s>>>(b.tlas, T, b.blas, B, d_xforms, b.nodes, b.d_state);
+        WB(cudaGetLastError());
+        WB(b.near_trees(a));
+        WB(b.read_state());
+        facts->huge = b.h.huge;
+        return cudaStreamSynchronize(s);
+    }();
+    if (b.second) cudaFree(b.second);
+    const cudaError_t f = cudaFree(a.base);
+    return e != cudaSuccess ? e : f;
+}
+
+}  // namespace orn

@@ -65,7 +65,7 @@ struct Pool {
 // NW warps per block, NS of them shading, P path slots, launch bounds for
 // MINB resident blocks per SM (the register cap), STEPS node visits per
 // traversal round.
-template <int SEM, bool COUNT, bool FAST, int NW, int NS, int P, int MINB, int STEPS>
+template <int SEM, bool COUNT, bool FAST, bool NEAR, int NW, int NS, int P, int MINB, int STEPS>
 __global__ void __launch_bounds__(32 * NW, MINB)
 wave_kernel(RenderLaunch p) {
     extern __shared__ __align__(16) unsigned char wave_smem[];
@@ -215,7 +215,7 @@ wave_kernel(RenderLaunch p) {
     if (warp >= (uint32_t)NS) {
         // traversal warps: their lanes' stacks are the first 32 * (NW - NS)
         // columns of the shared stack array
-        traversal_warp<COUNT, FAST, P, STEPS>(pool, p, sstack + (threadIdx.x - 32 * NS), 32 * (NW - NS), lane, vc,
+        traversal_warp<COUNT, FAST, NEAR, P, STEPS>(pool, p, sstack + (threadIdx.x - 32 * NS), 32 * (NW - NS), lane, vc,
                                               err);
     } else {
         // the shading warp: up to 32 queued hits per round
@@ -302,13 +302,13 @@ constexpr size_t shape_smem() {
     return ((sizeof(Pool<T::P>) + 15) / 16) * 16 + sizeof(uint32_t) * kSmemStack * 32 * (T::W - T::S);
 }
 
-template <int SEM, bool COUNT, bool FAST, int SHAPE, int STEPS>
+template <int SEM, bool COUNT, bool FAST, bool NEAR, int SHAPE, int STEPS>
 cudaError_t launch_wave_t(const RenderLaunch& p, cudaStream_t s) {
     using T = Shape<SHAPE>;
     constexpr int kBlock = 32 * T::W;
     constexpr size_t kSmem = shape_smem<SHAPE>();
     static int blocks_per_sm = 0, sms = 0;
-    auto kern = wave_kernel<SEM, COUNT, FAST, T::W, T::S, T::P, T::B, STEPS>;
+    auto kern = wave_kernel<SEM, COUNT, FAST, NEAR, T::W, T::S, T::P, T::B, STEPS>;
     // more than 48 KB of dynamic shared memory: an opt-in per device
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return e;
@@ -329,13 +329,13 @@ cudaError_t launch_wave_t(const RenderLaunch& p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template <int SEM, bool FAST, int STEPS>
+template <int SEM, bool FAST, bool NEAR, int STEPS>
 cudaError_t launch_wave_steps(const RenderLaunch& p, int shape, cudaStream_t s) {
     switch (shape) {
-        case 1: return launch_wave_t<SEM, false, FAST, 1, STEPS>(p, s);
-        case 2: return launch_wave_t<SEM, false, FAST, 2, STEPS>(p, s);
-        case 3: return launch_wave_t<SEM, false, FAST, 3, STEPS>(p, s);
-        default: return launch_wave_t<SEM, false, FAST, 0, STEPS>(p, s);
+        case 1: return launch_wave_t<SEM, false, FAST, NEAR, 1, STEPS>(p, s);
+        case 2: return launch_wave_t<SEM, false, FAST, NEAR, 2, STEPS>(p, s);
+        case 3: return launch_wave_t<SEM, false, FAST, NEAR, 3, STEPS>(p, s);
+        default: return launch_wave_t<SEM, false, FAST, NEAR, 0, STEPS>(p, s);
     }
 }
 
@@ -343,9 +343,12 @@ cudaError_t launch_wave_steps(const RenderLaunch& p, int shape, cudaStream_t s) 
 // steps per round only.
 template <int SEM, bool FAST>
 cudaError_t launch_wave_shape(const RenderLaunch& p, const WaveConfig& c, bool count, cudaStream_t s) {
-    if (count) return launch_wave_t<SEM, true, FAST, 0, 32>(p, s);
-    return c.steps == 64 ? launch_wave_steps<SEM, FAST, 64>(p, c.shape, s)
-                         : launch_wave_steps<SEM, FAST, 32>(p, c.shape, s);
+    if (count) return launch_wave_t<SEM, true, FAST, false, 0, 32>(p, s);
+    if (FAST && p.scene.near)
+        return c.steps == 64 ? launch_wave_steps<SEM, FAST, FAST, 64>(p, c.shape, s)
+                             : launch_wave_steps<SEM, FAST, FAST, 32>(p, c.shape, s);
+    return c.steps == 64 ? launch_wave_steps<SEM, FAST, false, 64>(p, c.shape, s)
+                         : launch_wave_steps<SEM, FAST, false, 32>(p, c.shape, s);
 }
 
 }  // namespace

@@ -207,14 +207,10 @@ wave_cached_kernel(RenderLaunch p) {
                     if (mtype > ORN_DIELECTRIC) {
                         // emitter (or unknown type): the path ends with color x emission,
                         // unless the previous vertex sampled this emitter directly
-                        const uint32_t etex = bits(ma.w);
-                        const bool etex_on = SEM == SEM_WGSL
-                                                 ? (etex < p.cp.textures_count && etex < p.scene.textures_len)
-                                                 : etex < p.scene.textures_len;
-                        f3 em = mk(0.0f, 0.0f, 0.0f);
-                        if (mtype == ORN_DIFFUSE_LIGHT)
-                            em = etex_on ? tex_sample(p.scene.textures[etex], g.hu, g.hv, SEM == SEM_WGSL)
-                                         : mk(ma.x, ma.y, ma.z);
+                        bool textured;
+                        const f3 em = mtype == ORN_DIFFUSE_LIGHT
+                                          ? surface_color<SEM, MATH_PORTABLE>(p.scene, p.cp, h, g, ma, &textured)
+                                          : mk(0.0f, 0.0f, 0.0f);
                         f3 c2 = mul(color, em);
                         const bool sampled = (pf & B_NEE_PREV) && h.type == ORN_NODE_MESH &&
                                              __ldg(p.cache.light_material + h.material) != 0u;
@@ -233,12 +229,8 @@ wave_cached_kernel(RenderLaunch p) {
                     } else {
                         const bool rough = mtype == ORN_LAMBERTIAN || (mtype == ORN_METAL && mb.x >= kCacheMinFuzz);
                         auto surface_att = [&]() -> f3 {
-                            const uint32_t tex_id = bits(ma.w);
-                            const bool use_tex = SEM == SEM_WGSL
-                                                     ? (tex_id < p.cp.textures_count && tex_id < p.scene.textures_len)
-                                                     : tex_id < p.scene.textures_len;
-                            return use_tex ? tex_sample(p.scene.textures[tex_id], g.hu, g.hv, SEM == SEM_WGSL)
-                                           : mk(ma.x, ma.y, ma.z);
+                            bool textured;
+                            return surface_color<SEM, MATH_PORTABLE>(p.scene, p.cp, h, g, ma, &textured);
                         };
                         bool at_cache = false;
                         f3 aclamp = mk(1.0f, 1.0f, 1.0f);

@@ -14,6 +14,9 @@
 #include "pt_kernels.h"
 #include "pt_device.cuh"
 #include "pt_machine.cuh"
+#include "pt_near.cuh"
+
+#include <type_traits>
 
 namespace orn {
 namespace wave {
@@ -242,11 +245,11 @@ __device__ __forceinline__ void wave_warp(Pool& pool, const RenderLaunch& p, uin
 // no shading code (measured: 331 against 274 Msamples/s for wave_warp with
 // the traversal-only role on the 1080p workload).  Returns when the block is
 // finished or a wait ran out.
-template <bool COUNT, bool FAST, int P, int STEPS, class Pool>
+template <bool COUNT, bool FAST, bool NEAR, int P, int STEPS, class Pool>
 __device__ __forceinline__ void traversal_warp(Pool& pool, const RenderLaunch& p, uint32_t* sstack, int stride,
                                                uint32_t lane, VisitCount& vc, uint32_t& err) {
     const unsigned kFull = 0xffffffffu;
-    TravStack<kSmemStack> stack;
+    TravStack<kSmemStack, NEAR ? kNearStackWords : kStackSize> stack;
     stack.sstack = sstack;
     stack.sstride = stride;
     const float t_min = p.cp.ray_cast_epsilon;
@@ -254,7 +257,7 @@ __device__ __forceinline__ void traversal_warp(Pool& pool, const RenderLaunch& p
     uint32_t slot = kEmpty, steps = 0;
     f3 ro = mk(0.0f, 0.0f, 0.0f), rd = ro;
     HitRec h;
-    Walker w;
+    std::conditional_t<NEAR, NearWalker, Walker> w;
     bool ok = true;
     uint64_t idle_since = 0;
     for (;;) {
@@ -296,18 +299,32 @@ __device__ __forceinline__ void traversal_warp(Pool& pool, const RenderLaunch& p
             // visits counted once per round, as in the megakernel
             uint32_t s = 0;
             const uint32_t e0 = err;
+            if constexpr (NEAR) {
+                // (a step of these is several visits; measured on the 1080p
+                // scene: STEPS per round 95 ms, STEPS / 8 83.5, STEPS / 16 85.6)
 #pragma unroll 1
-            while (s < (uint32_t)STEPS) {
-                ++s;
-                if (!walker_step<COUNT, kSmemStack, FAST, false, COUNT>(w, p.scene, ro, rd, t_min, &h, stack, &vc,
-                                                                        &err)) {
-                    fin = true;
-                    break;
+                while (s < (uint32_t)(STEPS / 8)) {
+                    ++s;
+                    if (!near_step(w, p.scene, ro, rd, t_min, stack)) {
+                        fin = true;
+                        break;
+                    }
                 }
+                if (fin) flag = near_finish(w, p.scene, &h) ? HIT_ANY : HIT_MISS;
+            } else {
+#pragma unroll 1
+                while (s < (uint32_t)STEPS) {
+                    ++s;
+                    if (!walker_step<COUNT, kSmemStack, FAST, false, COUNT>(w, p.scene, ro, rd, t_min, &h, stack, &vc,
+                                                                            &err)) {
+                        fin = true;
+                        break;
+                    }
+                }
+                if (!COUNT && !fin && !walker_account_round(w, s, &err)) fin = true;
+                if (fin) flag = err != e0 ? HIT_FAILED : (w.any ? HIT_ANY : HIT_MISS);
             }
             steps += s;
-            if (!COUNT && !fin && !walker_account_round(w, s, &err)) fin = true;
-            if (fin) flag = err != e0 ? HIT_FAILED : (w.any ? HIT_ANY : HIT_MISS);
         }
         if (fin) {
             pool.t[slot] = h.t;
