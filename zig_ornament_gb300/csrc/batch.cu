@@ -23,31 +23,37 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "batch.h"
 #include "pt_kernels.h"
 #include "pt_device.cuh"
 #include "pt_machine.cuh"
+#include "pt_near.cuh"
 #include "tune_cache.h"
 
 namespace orn {
 
 namespace {
 
-enum BatchLane { B_IDLE = 0, B_TRAVERSE = 1, B_SHADE = 2, B_DONE = 3 };
+enum BatchLane { B_IDLE = 0, B_TRAVERSE = 1, B_SHADE = 2, B_DONE = 3, B_START = 4 };
 
-// Resident blocks per SM each block size is compiled for (80 registers a
-// thread at 128 and 192).
-template <int BLOCK> constexpr int batch_min_blocks() { return BLOCK == 64 ? 8 : (BLOCK == 128 ? 6 : 4); }
+// Resident blocks per SM each block size is compiled for: 80 registers a
+// thread at 128 and 192; on the near-first trees, whose step spills 150 bytes
+// there, 96 or more (six scenes, 128 threads: 6 blocks 58.8 ms, 5 52.6).
+template <int BLOCK, bool NEAR> constexpr int batch_min_blocks() {
+    return BLOCK == 64 ? 8 : (BLOCK == 128 ? (NEAR ? 5 : 6) : (NEAR ? 3 : 4));
+}
 
-template <int SEM, bool FAST, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, batch_min_blocks<BLOCK>())
+// NEAR: every context has near-first trees (pt_near.cuh).
+template <int SEM, bool FAST, bool NEAR, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, batch_min_blocks<BLOCK, NEAR>())
 batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t total_pixels, uint32_t* work_counter,
              uint32_t* error, int shade_threshold) {
     __shared__ uint32_t sstack[kSmemStack * BLOCK];
     const BatchView* __restrict__ sv = views;
-    TravStack<kSmemStack> stack;
+    TravStack<kSmemStack, NEAR ? kNearStackWords : kStackSize> stack;
     stack.sstack = sstack + threadIdx.x;
     stack.sstride = BLOCK;
     const unsigned kFull = 0xffffffffu;
@@ -57,11 +63,12 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
     int mode = B_IDLE;
     bool exhausted = false;
     uint32_t sc = 0, gid = 0, k = 0, bounce = 0;
-    // the lane's scene as traversal sees it: walker_begin / walker_step read
-    // only the node array, the root and the triangle-test choice
+    // the lane's scene as traversal sees it: walker_begin and the steps read
+    // only the node array, the roots and the triangle-test choice
     SceneDev tsc;
     tsc.nodes = nullptr;
     tsc.root_ref = 0;
+    tsc.nroot = 0;
     tsc.exact_slabs = 0;
     tsc.watertight = 0;
     Rng rng{0};
@@ -69,7 +76,7 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
     f3 ro = mk(0.0f, 0.0f, 0.0f), rd = ro, color = ro;
     HitRec h;
     h.t = 0.0f; h.material = 0; h.type = 0; h.inv = 0; h.tri = 0; h.u = 0.0f; h.v = 0.0f;
-    Walker w;
+    std::conditional_t<NEAR, NearWalker, Walker> w;
     VisitCount vc = {0, 0, 0, 0, 0};
     SampleCount scn = {0, 0, 0, 0};
     uint32_t err = 0;
@@ -103,8 +110,10 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
     };
 
     for (;;) {
-        const unsigned idle = __ballot_sync(kFull, mode == B_IDLE);
-        if (idle != 0u && !exhausted) {
+        for (;;) {   // (one copy of start_samples, as in the megakernel)
+            if (mode == B_START) mode = start_samples();
+            const unsigned idle = __ballot_sync(kFull, mode == B_IDLE);
+            if (idle == 0u || exhausted) break;
             const unsigned leader = __ffs(idle) - 1u;
             const unsigned n = __popc(idle);
             uint32_t base = 0;
@@ -124,12 +133,13 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
                     sc = lo;
                     tsc.nodes = sv[sc].scene.nodes;
                     tsc.root_ref = sv[sc].scene.root_ref;
+                    tsc.nroot = sv[sc].scene.nroot;
                     tsc.watertight = sv[sc].scene.watertight;
                     gid = mine - sv[sc].pixel_begin;
                     rng.state = sv[sc].rng[gid];
                     acc = sv[sc].cp.current_iteration > 1.0f ? sv[sc].acc[gid] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     k = 0;
-                    mode = start_samples();
+                    mode = B_START;
                 }
             }
         }
@@ -140,11 +150,21 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
 
         if (mode == B_TRAVERSE) {
             const float t_min = sv[sc].cp.ray_cast_epsilon;
+            if constexpr (NEAR) {
 #pragma unroll 1
-            for (int s = 0; s < kStepsPerIteration; ++s) {
-                if (!walker_step<false, kSmemStack, FAST>(w, tsc, ro, rd, t_min, &h, stack, &vc, &err)) {
-                    mode = B_SHADE;
-                    break;
+                for (int s = 0; s < kNearSteps; ++s) {
+                    if (!near_step(w, tsc, ro, rd, t_min, stack)) {
+                        mode = B_SHADE;
+                        break;
+                    }
+                }
+            } else {
+#pragma unroll 1
+                for (int s = 0; s < kStepsPerIteration; ++s) {
+                    if (!walker_step<false, kSmemStack, FAST>(w, tsc, ro, rd, t_min, &h, stack, &vc, &err)) {
+                        mode = B_SHADE;
+                        break;
+                    }
                 }
             }
         }
@@ -154,8 +174,10 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
         if (ready != 0u && ((int)__popc(ready) >= shade_threshold || busy == 0u)) {
             if (mode == B_SHADE) {
                 const BatchView& V = sv[sc];
-                bool cont;
-                if (!w.any) {
+                bool cont, any;
+                if constexpr (NEAR) any = near_finish(w, tsc, &h);
+                else any = w.any;
+                if (!any) {
                     if (err) color = mk(0.0f, 0.0f, 0.0f);
                     else color = sky_color(color, rd);
                     cont = false;
@@ -168,7 +190,7 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
                 } else {
                     add_sample(V.cp.current_iteration + (float)k);
                     ++k;
-                    mode = start_samples();
+                    mode = B_START;
                 }
             }
         }
@@ -179,66 +201,74 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
 
 // SM count and resident blocks of one instantiation, queried once (the
 // first query runs before any stream capture: launch_frame primes it).
-template <int SEM, bool FAST, int BLOCK>
+template <int SEM, bool FAST, bool NEAR, int BLOCK>
 void occupancy(int* sms_out, int* maxb_out) {
     static int sms = 0, maxb = 0;
     if (sms == 0) {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, batch_kernel<SEM, FAST, BLOCK>, BLOCK, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, batch_kernel<SEM, FAST, NEAR, BLOCK>, BLOCK, 0);
     }
     *sms_out = sms;
     *maxb_out = maxb;
 }
 
-template <int SEM, bool FAST, int BLOCK>
+template <int SEM, bool FAST, bool NEAR, int BLOCK>
 cudaError_t launch_tt(const BatchView* views, uint32_t nviews, uint32_t total_pixels, uint32_t* work_counter,
                       uint32_t* error, const BatchConfig& cfg, cudaStream_t s) {
     int sms = 0, maxb = 0;
-    occupancy<SEM, FAST, BLOCK>(&sms, &maxb);
+    occupancy<SEM, FAST, NEAR, BLOCK>(&sms, &maxb);
     const int per_sm = std::max(1, std::min(cfg.blocks_per_sm, std::max(maxb, 1)));
     uint32_t grid = (uint32_t)(per_sm * sms);
     const uint32_t need = (total_pixels + BLOCK - 1) / BLOCK;
     if (need < grid) grid = std::max<uint32_t>(need, 1u);
-    batch_kernel<SEM, FAST, BLOCK><<<grid, BLOCK, 0, s>>>(views, nviews, total_pixels, work_counter, error,
+    batch_kernel<SEM, FAST, NEAR, BLOCK><<<grid, BLOCK, 0, s>>>(views, nviews, total_pixels, work_counter, error,
                                                            cfg.shade_threshold);
     return cudaGetLastError();
 }
 
-template <int SEM, bool FAST>
+template <int SEM, bool FAST, bool NEAR>
 cudaError_t launch_t(const BatchView* views, uint32_t nviews, uint32_t total_pixels, uint32_t* work_counter,
                      uint32_t* error, const BatchConfig& cfg, cudaStream_t s) {
     switch (cfg.block) {
-        case 64: return launch_tt<SEM, FAST, 64>(views, nviews, total_pixels, work_counter, error, cfg, s);
-        case 192: return launch_tt<SEM, FAST, 192>(views, nviews, total_pixels, work_counter, error, cfg, s);
-        default: return launch_tt<SEM, FAST, 128>(views, nviews, total_pixels, work_counter, error, cfg, s);
+        case 64: return launch_tt<SEM, FAST, NEAR, 64>(views, nviews, total_pixels, work_counter, error, cfg, s);
+        case 192: return launch_tt<SEM, FAST, NEAR, 192>(views, nviews, total_pixels, work_counter, error, cfg, s);
+        default: return launch_tt<SEM, FAST, NEAR, 128>(views, nviews, total_pixels, work_counter, error, cfg, s);
     }
 }
 
-template <int SEM, bool FAST>
+template <int SEM, bool FAST, bool NEAR>
 int max_blocks_t(int block) {
     int sms = 0, m = 0;
-    if (block == 64) occupancy<SEM, FAST, 64>(&sms, &m);
-    else if (block == 192) occupancy<SEM, FAST, 192>(&sms, &m);
-    else occupancy<SEM, FAST, 128>(&sms, &m);
+    if (block == 64) occupancy<SEM, FAST, NEAR, 64>(&sms, &m);
+    else if (block == 192) occupancy<SEM, FAST, NEAR, 192>(&sms, &m);
+    else occupancy<SEM, FAST, NEAR, 128>(&sms, &m);
     return m;
 }
 
 }  // namespace
 
 cudaError_t launch_batch(const BatchView* views, uint32_t nviews, uint32_t total_pixels, uint32_t* work_counter,
-                         uint32_t* error, int semantics, bool fast, const BatchConfig& cfg, cudaStream_t s) {
+                         uint32_t* error, int semantics, int slabs, const BatchConfig& cfg, cudaStream_t s) {
+    auto go = [&](auto f) { return f(views, nviews, total_pixels, work_counter, error, cfg, s); };
     if (semantics == SEM_WGSL)
-        return fast ? launch_t<SEM_WGSL, true>(views, nviews, total_pixels, work_counter, error, cfg, s)
-                    : launch_t<SEM_WGSL, false>(views, nviews, total_pixels, work_counter, error, cfg, s);
-    return fast ? launch_t<SEM_HIP, true>(views, nviews, total_pixels, work_counter, error, cfg, s)
-                : launch_t<SEM_HIP, false>(views, nviews, total_pixels, work_counter, error, cfg, s);
+        return slabs == BATCH_NEAR ? go(launch_t<SEM_WGSL, true, true>)
+                                   : (slabs == BATCH_FAST ? go(launch_t<SEM_WGSL, true, false>)
+                                                          : go(launch_t<SEM_WGSL, false, false>));
+    return slabs == BATCH_NEAR ? go(launch_t<SEM_HIP, true, true>)
+                               : (slabs == BATCH_FAST ? go(launch_t<SEM_HIP, true, false>)
+                                                      : go(launch_t<SEM_HIP, false, false>));
 }
 
-int batch_max_blocks_per_sm(int block, int semantics, bool fast) {
-    if (semantics == SEM_WGSL) return fast ? max_blocks_t<SEM_WGSL, true>(block) : max_blocks_t<SEM_WGSL, false>(block);
-    return fast ? max_blocks_t<SEM_HIP, true>(block) : max_blocks_t<SEM_HIP, false>(block);
+int batch_max_blocks_per_sm(int block, int semantics, int slabs) {
+    if (semantics == SEM_WGSL)
+        return slabs == BATCH_NEAR ? max_blocks_t<SEM_WGSL, true, true>(block)
+                                   : (slabs == BATCH_FAST ? max_blocks_t<SEM_WGSL, true, false>(block)
+                                                          : max_blocks_t<SEM_WGSL, false, false>(block));
+    return slabs == BATCH_NEAR ? max_blocks_t<SEM_HIP, true, true>(block)
+                               : (slabs == BATCH_FAST ? max_blocks_t<SEM_HIP, true, false>(block)
+                                                      : max_blocks_t<SEM_HIP, false, false>(block));
 }
 
 }  // namespace orn
@@ -260,7 +290,7 @@ struct orn_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint32_t g_nviews = 0, g_pixels = 0, g_sem = 0;
-    bool g_fast = false;
+    int g_slabs = 0;
     orn::BatchConfig g_cfg{0, 0, 0};
     bool rendered = false;
     uint64_t frames = 0;
@@ -291,9 +321,9 @@ void drop_graph(orn_batch* b) {
 
 // Host side of one frame: every context's orn_render bookkeeping, the view
 // table (pinned) and the frame's pixel total.
-int prepare_frame(orn_batch* b, uint32_t* total_pixels, uint32_t* semantics, bool* fast) {
+int prepare_frame(orn_batch* b, uint32_t* total_pixels, uint32_t* semantics, int* slabs) {
     uint64_t total = 0;
-    bool all_fast = true;
+    int all = orn::BATCH_NEAR;
     uint32_t sem0 = 0;
     for (size_t i = 0; i < b->contexts.size(); ++i) {
         orn::BatchView v;
@@ -308,33 +338,33 @@ int prepare_frame(orn_batch* b, uint32_t* total_pixels, uint32_t* semantics, boo
         v.pixel_begin = (uint32_t)total;
         total += (uint64_t)v.cp.width * v.cp.height;
         if (total >= 0xFFFFFFFFull) return bfail(b, ORN_ERR_INVALID_ARGUMENT, "batch frame too large");
-        all_fast = all_fast && f;
+        all = std::min<int>(all, !f ? orn::BATCH_EXACT : (v.scene.near ? orn::BATCH_NEAR : orn::BATCH_FAST));
         b->h_views[i] = v;
     }
     *total_pixels = (uint32_t)total;
     *semantics = sem0;
-    *fast = all_fast;
+    *slabs = all;
     return ORN_OK;
 }
 
 // Queues one frame: the view table, the work counter and the kernel, from a
 // CUDA graph captured for this (view count, pixel total, semantics, slab
 // mode, launch shape) and replayed afterwards.
-int launch_frame(orn_batch* b, uint32_t nviews, uint32_t total, uint32_t sem, bool fast) {
+int launch_frame(orn_batch* b, uint32_t nviews, uint32_t total, uint32_t sem, int slabs) {
     const orn::BatchConfig& c = b->config;
     const bool same = b->exec && b->g_nviews == nviews && b->g_pixels == total && b->g_sem == sem &&
-                      b->g_fast == fast && b->g_cfg.block == c.block && b->g_cfg.blocks_per_sm == c.blocks_per_sm &&
+                      b->g_slabs == slabs && b->g_cfg.block == c.block && b->g_cfg.blocks_per_sm == c.blocks_per_sm &&
                       b->g_cfg.shade_threshold == c.shade_threshold;
     if (!same) {
         drop_graph(b);
         // the launcher's device queries happen here, outside the capture
-        orn::batch_max_blocks_per_sm(c.block, (int)sem, fast);
+        orn::batch_max_blocks_per_sm(c.block, (int)sem, slabs);
         B_CUDA(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = cudaMemcpyAsync(b->d_views, b->h_views, nviews * sizeof(orn::BatchView),
                                         cudaMemcpyHostToDevice, b->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(b->d_work, 0, 4, b->stream);
         if (e == cudaSuccess)
-            e = orn::launch_batch(b->d_views, nviews, total, b->d_work, b->d_error, (int)sem, fast, c, b->stream);
+            e = orn::launch_batch(b->d_views, nviews, total, b->d_work, b->d_error, (int)sem, slabs, c, b->stream);
         cudaGraph_t g = nullptr;
         cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
         if (e != cudaSuccess || e2 != cudaSuccess) {
@@ -347,7 +377,7 @@ int launch_frame(orn_batch* b, uint32_t nviews, uint32_t total, uint32_t sem, bo
         b->g_nviews = nviews;
         b->g_pixels = total;
         b->g_sem = sem;
-        b->g_fast = fast;
+        b->g_slabs = slabs;
         b->g_cfg = c;
     }
     B_CUDA(b, cudaGraphLaunch(b->exec, b->stream));
@@ -438,11 +468,11 @@ int orn_batch_render(orn_batch* b) {
     // the previous frame has read the pinned view table before it is rewritten
     B_CUDA(b, cudaEventSynchronize(b->ev_done));
     uint32_t total = 0, sem = 0;
-    bool fast = false;
-    int st = prepare_frame(b, &total, &sem, &fast);
+    int slabs = 0;
+    int st = prepare_frame(b, &total, &sem, &slabs);
     if (st) return st;
     B_CUDA(b, cudaEventRecord(b->ev_start, b->stream));
-    st = launch_frame(b, (uint32_t)b->contexts.size(), total, sem, fast);
+    st = launch_frame(b, (uint32_t)b->contexts.size(), total, sem, slabs);
     if (st) return st;
     B_CUDA(b, cudaEventRecord(b->ev_stop, b->stream));
     B_CUDA(b, cudaEventRecord(b->ev_done, b->stream));
@@ -504,7 +534,7 @@ int orn_batch_tune(orn_batch* b, const char* cache_path, orn_batch_config* chose
     // per context: the contexts' own images and progress are untouched.
     std::vector<orn::BatchView> saved(b->contexts.size());
     uint64_t total64 = 0, samples = 0;
-    bool fast = true;
+    int slabs = orn::BATCH_NEAR;
     uint32_t sem = 0;
     for (size_t i = 0; i < b->contexts.size(); ++i) {
         bool f = false;
@@ -512,7 +542,7 @@ int orn_batch_tune(orn_batch* b, const char* cache_path, orn_batch_config* chose
         int dev = 0;
         int st = orn::batch_prepare(b->contexts[i], &saved[i], &f, &sm, &dev, b->stream, false);
         if (st) return bfail(b, st, orn_last_error(b->contexts[i]));
-        fast = fast && f;
+        slabs = std::min<int>(slabs, !f ? orn::BATCH_EXACT : (saved[i].scene.near ? orn::BATCH_NEAR : orn::BATCH_FAST));
         sem = sm;
         const uint32_t px = saved[i].cp.width * saved[i].cp.height;
         saved[i].pixel_begin = (uint32_t)total64;
@@ -527,7 +557,7 @@ int orn_batch_tune(orn_batch* b, const char* cache_path, orn_batch_config* chose
         std::snprintf(dev_name, sizeof(dev_name), "%s", prop.name);
     char key[512];
     std::snprintf(key, sizeof(key), "%s|sm%d|scenes=%zu|pixels=%u|samples=%llu|sem=%u|fast=%d", dev_name, b->sms,
-                  b->contexts.size(), total, (unsigned long long)samples, sem, fast ? 1 : 0);
+                  b->contexts.size(), total, (unsigned long long)samples, sem, slabs);
     auto cache = read_cache(cache_path);
     auto hit = cache.find(key);
     if (hit != cache.end()) {
@@ -564,7 +594,7 @@ int orn_batch_tune(orn_batch* b, const char* cache_path, orn_batch_config* chose
     float best_ms = 3.0e38f;
     int st = ORN_OK;
     for (int bi = 0; bi < 3 && st == ORN_OK; ++bi) {
-        const int maxb = orn::batch_max_blocks_per_sm(blocks[bi], (int)sem, fast);
+        const int maxb = orn::batch_max_blocks_per_sm(blocks[bi], (int)sem, slabs);
         if (maxb < 1) continue;
         const int fracs[3] = {maxb, std::max(1, (3 * maxb) / 4), std::max(1, maxb / 2)};
         for (int fi = 0; fi < 3 && st == ORN_OK; ++fi) {
@@ -578,7 +608,7 @@ int orn_batch_tune(orn_batch* b, const char* cache_path, orn_batch_config* chose
                     if (e == cudaSuccess) e = cudaEventRecord(b->ev_start, b->stream);
                     if (e == cudaSuccess)
                         e = orn::launch_batch(b->d_views, (uint32_t)saved.size(), total, b->d_work, b->d_error,
-                                              (int)sem, fast, c, b->stream);
+                                              (int)sem, slabs, c, b->stream);
                     if (e == cudaSuccess) e = cudaEventRecord(b->ev_stop, b->stream);
                     if (e == cudaSuccess) e = cudaEventSynchronize(b->ev_stop);
                     if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, b->ev_start, b->ev_stop);

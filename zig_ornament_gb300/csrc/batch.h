@@ -40,10 +40,14 @@ struct BatchConfig {
     int shade_threshold; // ready lanes needed before a warp shades
 };
 
+// What every context of a batch allows: the exact slab test only, the FMNMX
+// form, or the near-first trees (which imply that form).
+enum { BATCH_EXACT = 0, BATCH_FAST = 1, BATCH_NEAR = 2 };
+
 // Launches one batched frame (views already in device memory).
 cudaError_t launch_batch(const BatchView* views, uint32_t nviews, uint32_t total_pixels, uint32_t* work_counter,
-                         uint32_t* error, int semantics, bool fast, const BatchConfig& cfg, cudaStream_t s);
+                         uint32_t* error, int semantics, int slabs, const BatchConfig& cfg, cudaStream_t s);
 // The largest resident block count per SM for a block size (0 if unknown).
-int batch_max_blocks_per_sm(int block, int semantics, bool fast);
+int batch_max_blocks_per_sm(int block, int semantics, int slabs);
 
 }  // namespace orn
