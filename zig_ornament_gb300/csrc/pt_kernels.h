@@ -48,6 +48,16 @@ constexpr int kNearSteps = ORN_NEAR_STEPS;
 #endif
 constexpr int kNearInner = ORN_NEAR_INNER;
 
+// Ray lists (trace_near_kernel): idle lanes a warp gathers before it takes new
+// rays, and steps between looks at them.
+#ifndef ORN_TRACE_FETCH
+#define ORN_TRACE_FETCH 8
+#endif
+#ifndef ORN_TRACE_STEPS
+#define ORN_TRACE_STEPS 4
+#endif
+constexpr int kTraceFetch = ORN_TRACE_FETCH, kTraceSteps = ORN_TRACE_STEPS;
+
 // Radiance-cache side of a cached megakernel launch.  Every pixel traces one
 // sample, with next-event estimation: at a lambertian vertex whose scattered
 // ray will be traced, a point on an emissive mesh triangle is sampled by area
@@ -137,6 +147,7 @@ struct RenderLaunch {
     const uint32_t* order;     // hand-out order of the pixels (null: raster order)
     uint32_t* cost;            // per-pixel traversal steps of this launch (or null)
     int wave_fetch;            // wavefront kernels: idle lanes a traversing warp gathers before taking rays
+    uint32_t lanes;            // megakernel: lanes of a warp that take pixels (set by its launcher)
 };
 
 // Launch parameters of the persistent wavefront (wave.cu): one of the
@@ -270,8 +281,13 @@ cudaError_t launch_wave(const RenderLaunch& p, const WaveConfig& c, int semantic
 cudaError_t launch_wf_logic(const WaveLaunch& p, uint32_t iter, int semantics, int math, bool count,
                             cudaStream_t s);
 cudaError_t launch_wf_extend(const WaveLaunch& p, uint32_t iter, bool count, bool fast, cudaStream_t s);
+// Closest hits of a ray list: the reference's walk, with visits when asked
+// for; or, with `work` (count + 2 words of working memory, for scenes with
+// near-first trees and fewer than 2^32 - 1 rays), on those trees; `all_safe`:
+// every ray fits the FMNMX slab test.
 cudaError_t launch_trace_rays(const SceneDev& sc, float t_min, const float* rays, size_t count,
-                              orn_hit* hits, uint32_t* visits, uint32_t* error, cudaStream_t s);
+                              orn_hit* hits, uint32_t* visits, uint32_t* error, uint32_t* work, bool all_safe,
+                              cudaStream_t s);
 cudaError_t launch_seed_rng(uint32_t* rng, uint32_t n, cudaStream_t s, uint32_t first = 0);   // rng[i] = first + i
 cudaError_t launch_post(const float4* acc, float4* fb, uint32_t W, uint32_t H, uint32_t flip_y,
                         float ci, float inv_gamma, int semantics, int math, cudaStream_t s);
