@@ -588,13 +588,12 @@ int build_all(const orn_scene_desc* d, orn_bvh* b) {
             return d->meshes[a].vertex_indices_len > d->meshes[c].vertex_indices_len;
         });
         if (d->builder == ORN_BVH_LBVH) {
-            // on the GPU, one mesh after another
-            for (uint32_t i = 0; i < M; ++i) {
-                const size_t nt = d->meshes[i].vertex_indices_len / 3;
-                int st = orn::lbvh_build_blas(tris[i].v.data(), (uint32_t)nt, tris[i].first_global,
-                                              (uint32_t)blas_base[i], b->blas.data() + blas_base[i]);
-                if (st != ORN_OK) return st;
-            }
+            std::vector<orn::LbvhJob> jobs(M);
+            for (uint32_t i = 0; i < M; ++i)
+                jobs[i] = orn::LbvhJob{tris[i].v.data(), d->meshes[i].vertex_indices_len / 3, tris[i].first_global,
+                                       (uint32_t)blas_base[i], b->blas.data() + blas_base[i]};
+            const int st = orn::lbvh_build_all(jobs.data(), jobs.size());
+            if (st != ORN_OK) return st;
             order.clear();
         }
         std::atomic_size_t cursor{0};

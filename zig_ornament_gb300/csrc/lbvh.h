@@ -8,11 +8,17 @@
 
 namespace orn {
 
-// Builds the BLAS of one mesh on the current CUDA device: `tri_host` holds
-// n triangles as 9 floats (v0, v1, v2, object space); writes 2n - 1 nodes to
-// out_host in the reference's format (post-order, root last; child ids are
-// node_offset + slot, triangle ids first_global + index).  Returns ORN_*.
-int lbvh_build_blas(const float* tri_host, uint32_t n, uint32_t first_global, uint32_t node_offset,
-                    orn_bvh_node* out_host);
+// One mesh: `tri` holds n triangles as 9 floats (v0, v1, v2, object space);
+// its 2n - 1 nodes go to `out` in the reference's format (post-order, root
+// last; child ids are node_offset + slot, triangle ids first_global + index).
+struct LbvhJob {
+    const float* tri;
+    uint32_t n;
+    uint32_t first_global, node_offset;
+    orn_bvh_node* out;
+};
+
+// Builds the BLASes of `count` meshes on the current CUDA device.  Returns ORN_*.
+int lbvh_build_all(const LbvhJob* jobs, size_t count);
 
 }  // namespace orn

@@ -581,7 +581,7 @@ class Bvh:
                 if n == 0:
                     return np.zeros((0,) + shape, dtype=dtype)
                 nbytes = n * np.dtype(dtype).itemsize * int(np.prod(shape) if shape else 1)
-                raw = C.string_at(ptr, nbytes)
+                raw = (C.c_ubyte * nbytes).from_address(ptr)
                 return np.frombuffer(raw, dtype=dtype).reshape((n,) + shape).copy()
 
             self.tlas_nodes = arr(blob.tlas_nodes, blob.tlas_nodes_len, NODE_DTYPE, ())
