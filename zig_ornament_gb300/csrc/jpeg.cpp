@@ -18,7 +18,9 @@
 // (A.2).
 #include <algorithm>
 #include <cstring>
+#include <new>
 #include <string>
+#include <utility>
 
 #include "jpeg.h"
 #include "ornament_cuda.h"
@@ -44,6 +46,7 @@ struct Zigzag {
 const Zigzag kZigzag;
 
 constexpr int kFastBits = 9;
+constexpr int kPairBits = 11;
 
 struct Huffman {
     bool present = false;
@@ -52,6 +55,9 @@ struct Huffman {
     int32_t mincode[17] = {};
     int32_t valptr[17] = {};
     uint16_t fast[1 << kFastBits] = {};   // (length << 8) | symbol; 0: longer than kFastBits
+    // AC coefficients whose code and value bits fit kPairBits together:
+    // (value << 16) | (run << 8) | bits taken; 0: others
+    int32_t pair[1 << kPairBits] = {};
 
     bool build(const uint8_t counts[16], const uint8_t* symbols, int total) {
         std::memset(fast, 0, sizeof(fast));
@@ -78,10 +84,25 @@ struct Huffman {
             if (code > (1 << l)) return false;   // more codes than fit in l bits
             code <<= 1;
         }
+        for (uint32_t b = 0; b < (1u << kPairBits); ++b) {
+            const uint16_t f = fast[b >> (kPairBits - kFastBits)];
+            const int size = f & 15, bits = (f >> 8) + size;
+            pair[b] = 0;
+            if (f == 0 || size == 0 || size > 10 || bits > kPairBits) continue;
+            const int v = (int)((b >> (kPairBits - bits)) & ((1u << size) - 1u));
+            const int value = v < (1 << (size - 1)) ? v - (1 << size) + 1 : v;
+            pair[b] = (int32_t)(((uint32_t)value << 16) | ((uint32_t)((f & 0xFF) >> 4) << 8) | (uint32_t)bits);
+        }
         present = true;
         return true;
     }
 };
+
+// Whether one of the eight bytes is FF (a byte of the complement is zero).
+inline bool has_ff(uint64_t w) {
+    const uint64_t z = ~w;
+    return ((z - 0x0101010101010101ull) & ~z & 0x8080808080808080ull) != 0;
+}
 
 // Entropy-coded segment reader: byte stuffing (FF 00) removed, fill bytes
 // before a marker skipped, zeros fed once a marker or the end is reached.
@@ -93,7 +114,25 @@ struct Bits {
     bool at_marker = false;
     uint32_t zeros_fed = 0;
 
+    // Fills the buffer to more than 56 bits.
     void fill() {
+        const int k = (64 - cnt) >> 3;   // bytes that fit
+        if (k == 0) return;
+        if (!at_marker && end - p >= 8) {
+            uint64_t w;
+            std::memcpy(&w, p, 8);
+            w = __builtin_bswap64(w);                              // first byte on top
+            w &= ~(uint64_t)0 << (64 - 8 * k);
+            if (!has_ff(w)) {
+                buf |= w >> cnt;
+                p += k;
+                cnt += 8 * k;
+                return;
+            }
+        }
+        fill_bytes();
+    }
+    void fill_bytes() {
         while (cnt <= 56) {
             uint32_t b = 0;
             bool real = false;
@@ -161,33 +200,46 @@ inline int receive_extend(Bits& br, int s) {
     return v < (1 << (s - 1)) ? v - (1 << s) + 1 : v;
 }
 
-bool decode_block(Bits& br, const Huffman& dc, const Huffman& ac, int* pred, int16_t* out) {
-    std::memset(out, 0, 64 * sizeof(int16_t));
+// Writes the block's nonzero coefficients to `out` (room for 64); their
+// number, or -1 for corrupt data.
+int decode_block(Bits& br, const Huffman& dc, const Huffman& ac, int* pred, uint32_t* out) {
+    int n = 0;
     const int t = decode_symbol(br, dc);
-    if (t < 0 || t > 11) return false;
+    if (t < 0 || t > 11) return -1;
     br.fill();
     const int dcv = *pred + receive_extend(br, t);
-    if (dcv < -32768 || dcv > 32767) return false;
+    if (dcv < -32768 || dcv > 32767) return -1;
     *pred = dcv;
-    out[0] = (int16_t)dcv;
+    if (dcv != 0) out[n++] = entry_of(0, dcv);
     for (int k = 1; k < 64;) {
+        br.fill();
+        // a short code and its value with one look (not the block's last
+        // place, where the buffer is filled between the two)
+        const int32_t pr = ac.pair[br.peek(kPairBits)];
+        const int at = k + ((pr >> 8) & 15);
+        if (pr != 0 && at < 63) {
+            br.skip(pr & 0xFF);
+            out[n++] = entry_of(kZigzag.natural[at], pr >> 16);
+            k = at + 1;
+            continue;
+        }
         const int rs = decode_symbol(br, ac);
-        if (rs < 0) return false;
+        if (rs < 0) return -1;
         const int r = rs >> 4, s = rs & 15;
         if (s == 0) {
             if (r != 15) break;   // EOB
             k += 16;              // ZRL
-            if (k > 64) return false;
+            if (k > 64) return -1;
             continue;
         }
-        if (s > 10) return false;
+        if (s > 10) return -1;
         k += r;
-        if (k > 63) return false;
+        if (k > 63) return -1;
         br.fill();
-        out[kZigzag.natural[k]] = (int16_t)receive_extend(br, s);
+        out[n++] = entry_of(kZigzag.natural[k], receive_extend(br, s));
         ++k;
     }
-    return true;
+    return n;
 }
 
 struct Parser {
@@ -209,6 +261,20 @@ struct Parser {
     bool need(size_t n) const { return pos + n <= len; }
     uint32_t u8(size_t at) const { return data[at]; }
     uint32_t u16(size_t at) const { return ((uint32_t)data[at] << 8) | data[at + 1]; }
+
+    // Room for at least one more block's entries.  (Twice a coded byte's worth
+    // of entries to begin with; a start has to fit 32 bits, which 64 entries
+    // for each block of 2^28 pixels and several scans could exceed.)
+    bool more_room() {
+        const size_t room = img->entry_room ? 2 * img->entry_room : std::max<size_t>(2 * len, 4096);
+        if (room > 0xFFFFFFFFull) return false;
+        std::unique_ptr<uint32_t[]> p(new (std::nothrow) uint32_t[room]);
+        if (!p) return false;
+        if (img->entry_count) std::memcpy(p.get(), img->entries.get(), img->entry_count * 4);
+        img->entries = std::move(p);
+        img->entry_room = room;
+        return true;
+    }
 
     int read_dqt(size_t seg, size_t seg_len) {
         size_t at = seg, end = seg + seg_len;
@@ -284,15 +350,18 @@ struct Parser {
         if (img->ncomp == 3 && img->comp[0].id == 'R' && img->comp[1].id == 'G' && img->comp[2].id == 'B')
             img->ycbcr = false;
         if (!header_only) {
+            size_t total = 0;
             for (uint32_t i = 0; i < img->ncomp; ++i) {
                 Component& c = img->comp[i];
                 c.bw = img->mcux * c.h;
                 c.bh = img->mcuy * c.v;
-                try {
-                    c.coef.assign((size_t)c.bw * c.bh * 64, 0);
-                } catch (...) {
-                    return fail(ORN_ERR_OUT_OF_MEMORY, "out of host memory for the coefficients");
-                }
+                c.first_block = total;
+                total += (size_t)c.bw * c.bh;
+            }
+            try {
+                img->blocks.assign(total, Block{0, 0});
+            } catch (...) {
+                return fail(ORN_ERR_OUT_OF_MEMORY, "out of host memory for the coefficients");
             }
         }
         have_frame = true;
@@ -360,9 +429,13 @@ struct Parser {
                 for (uint32_t by = 0; by < nv; ++by)
                     for (uint32_t bx = 0; bx < nh; ++bx) {
                         const uint32_t col = mx * nh + bx, row = my * nv + by;
-                        int16_t* out = c.coef.data() + ((size_t)row * c.bw + col) * 64;
-                        if (!decode_block(br, dc[td[i]], ac[ta[i]], &pred[i], out))
-                            return fail(ORN_ERR_BAD_IMAGE, "corrupt entropy-coded data");
+                        if (img->entry_room - img->entry_count < 64 && !more_room())
+                            return fail(ORN_ERR_OUT_OF_MEMORY, "out of host memory for the coefficients");
+                        const int n = decode_block(br, dc[td[i]], ac[ta[i]], &pred[i],
+                                                   img->entries.get() + img->entry_count);
+                        if (n < 0) return fail(ORN_ERR_BAD_IMAGE, "corrupt entropy-coded data");
+                        img->blocks[c.first_block + (size_t)row * c.bw + col] = Block{(uint32_t)img->entry_count, (uint32_t)n};
+                        img->entry_count += (size_t)n;
                     }
             }
             if (br.zeros_fed > 64) return fail(ORN_ERR_BAD_IMAGE, "entropy-coded data ends early");
@@ -487,11 +560,19 @@ int orn_jpeg_coefficients(const void* data, size_t len, uint32_t component, int1
     if (blocks_h) *blocks_h = c.bh;
     if (quant) std::memcpy(quant, img.quant[c.tq], 64 * sizeof(uint16_t));
     if (out) {
-        if (out_len < c.coef.size()) {
+        const size_t plane = (size_t)c.bw * c.bh;
+        if (out_len < plane * 64) {
             last_error() = "coefficient buffer too small";
             return ORN_ERR_BUFFER_TOO_SMALL;
         }
-        std::memcpy(out, c.coef.data(), c.coef.size() * sizeof(int16_t));
+        std::memset(out, 0, plane * 64 * sizeof(int16_t));
+        for (size_t k = 0; k < plane; ++k) {
+            const Block& b = img.blocks[c.first_block + k];
+            for (uint32_t e = 0; e < b.count; ++e) {
+                const uint32_t v = img.entries[b.start + e];
+                out[k * 64 + (v >> 16)] = (int16_t)(uint16_t)v;
+            }
+        }
     }
     return ORN_OK;
 }

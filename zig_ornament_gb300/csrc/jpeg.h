@@ -11,6 +11,7 @@
 
 #include <stdint.h>
 
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -25,8 +26,18 @@ struct Component {
     uint32_t tq = 0;             // quantisation table
     uint32_t bw = 0, bh = 0;     // coefficient plane in 8x8 blocks (MCU-padded)
     bool decoded = false;
-    std::vector<int16_t> coef;   // [bh][bw][64], natural (row-major) order, not dequantised
+    size_t first_block = 0;      // of the plane in Image::blocks, [bh][bw]
 };
+
+// A block's nonzero coefficients: entries [start, start + count) of
+// Image::entries (a photograph has some six in 64: the planes written out
+// would be ten times the size, on the host, on the way and on the GPU).
+struct Block {
+    uint32_t start;
+    uint32_t count;
+};
+// natural (row-major) index << 16 | value as 16 bits, not dequantised
+inline uint32_t entry_of(int index, int value) { return ((uint32_t)index << 16) | (uint16_t)(int16_t)value; }
 
 struct Image {
     uint32_t width = 0, height = 0, ncomp = 0;
@@ -36,6 +47,9 @@ struct Image {
     Component comp[kMaxComponents];
     uint16_t quant[4][64] = {};  // natural order
     bool quant_present[4] = {};
+    std::vector<Block> blocks;   // all components' planes, one after another
+    std::unique_ptr<uint32_t[]> entries;
+    size_t entry_count = 0, entry_room = 0;
 };
 
 // Status codes are the library's ORN_* values.  With header_only the scan
