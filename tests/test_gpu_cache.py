@@ -61,6 +61,27 @@ def test_gradients_match_oracle():
     cache.close()
 
 
+# one row short of, at and past a tile; and past the tiles that the chip has in
+# flight at once (152 SMs x 3 tiles of 128), so that a group takes a second one
+# and a weight-gradient block sums several.  The bounds are those of the two
+# tests above: the roundings are the same at every size.
+@pytest.mark.parametrize("n", [127, 128, 129, 3 * 152 * 128 + 129])
+def test_edges_of_tiles(n):
+    cache = ornament.RadianceCache(seed=21)
+    p = cache.params()
+    x, t = _samples(n, n)
+    y_em, _, _ = rco.forward(p, x, emulate=True)
+    for m in (1, n):
+        y = cache.infer(x[:m]).astype(np.float64)
+        assert np.linalg.norm(y - y_em[:m]) < 5e-3 * np.linalg.norm(y_em[:m])
+    l_em, g_em = rco.loss_and_grads(p, x, t, emulate=True)
+    for _ in range(2):   # the second from cleared sums
+        g, loss = cache.gradients(x, t)
+        assert loss == pytest.approx(l_em, rel=2e-2)
+        assert max(_layer_errors(g, g_em)) < 2e-2
+    cache.close()
+
+
 def test_adam_step_matches_oracle():
     cache = ornament.RadianceCache(seed=13)
     p0 = cache.params()

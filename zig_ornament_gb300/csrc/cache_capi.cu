@@ -42,10 +42,13 @@ uint64_t splitmix(uint64_t& x) {
 }
 
 void free_buffers(orn_cache* c) {
-    void* ptrs[] = {c->params, c->m,  c->v,     c->grads, c->w_f16,  c->w_bf16,    c->d_loss, c->d_status,
-                    c->h,      c->dz, c->dz6,   c->io_in, c->io_target, c->io_out};
+    // (the loss and the status lie behind the gradients)
+    void* ptrs[] = {c->params, c->m,  c->v,   c->grads, c->w_f16,     c->w_bf16,
+                    c->h,      c->dz, c->dz6, c->io_in, c->io_target, c->io_out};
     for (void* p : ptrs)
         if (p) cudaFree(p);
+    if (c->host) cudaFreeHost(c->host);
+    c->host = nullptr;
     c->params = c->m = c->v = c->grads = nullptr;
     c->w_f16 = c->w_bf16 = nullptr;
     c->d_loss = nullptr;
@@ -102,10 +105,17 @@ int refresh_copies(orn_cache* c, cudaStream_t s) {
     return ORN_OK;
 }
 
-int finish(orn_cache* c) {
+// Waits for the stream's work.  The status comes back behind it in the same
+// copy as the loss and, with `grads` (which it then clears for the next step),
+// the gradients, into pinned memory (c->host), so that a call waits once.
+int finish(orn_cache* c, bool grads = false) {
+    const size_t from = grads ? 0 : orn::kWeightCount;
+    RC_CUDA(c, cudaMemcpyAsync(c->host + from, c->grads + from, (orn::kWeightCount + 2 - from) * 4,
+                               cudaMemcpyDeviceToHost, c->stream));
+    if (grads) RC_CUDA(c, cudaMemsetAsync(c->grads, 0, (size_t)orn::kWeightCount * 4, c->stream));
     RC_CUDA(c, cudaStreamSynchronize(c->stream));
     uint32_t st = 0;
-    RC_CUDA(c, cudaMemcpy(&st, c->d_status, 4, cudaMemcpyDeviceToHost));
+    std::memcpy(&st, c->host + orn::kWeightCount + 1, 4);
     if (st) {
         RC_CUDA(c, cudaMemset(c->d_status, 0, 4));
         return cfail(c, ORN_ERR_TIMEOUT, "a tensor-core wait timed out");
@@ -130,19 +140,13 @@ int cache_train_step(orn_cache* c, const float* d_in, const float* d_target, uin
     f.inputs = d_in;
     f.targets = d_target;
     f.h_out = c->h;
-    f.dz_out = c->dz6;
+    f.weights_bf16 = c->w_bf16;
+    f.dz6 = c->dz6;
+    f.dz = c->dz;
     f.loss = c->d_loss;
     f.n = n;
     f.status = status;
     RC_CUDA(c, rc_launch_forward(f, true, grid, s));
-    RcBackward b{};
-    b.weights_bf16 = c->w_bf16;
-    b.dz6 = c->dz6;
-    b.h = c->h;
-    b.dz = c->dz;
-    b.n = n;
-    b.status = status;
-    RC_CUDA(c, rc_launch_backward(b, grid, s));
     RcWgrad g{};
     g.inputs = d_in;
     g.h = c->h;
@@ -150,7 +154,10 @@ int cache_train_step(orn_cache* c, const float* d_in, const float* d_target, uin
     g.dz6 = c->dz6;
     g.grads = c->grads;
     g.n = n;
-    g.splits = std::min<uint32_t>(tiles, 32u);
+    // every CTA resident at once, each with the same number of tiles
+    const uint32_t resident = std::max(1u, (uint32_t)(c->sms * kWgradPerSm / kWgradJobs));
+    const uint32_t rounds = (tiles + resident - 1) / resident;
+    g.splits = (tiles + rounds - 1) / rounds;
     g.status = status;
     RC_CUDA(c, rc_launch_wgrad(g, s));
     if (adam) {
@@ -239,11 +246,13 @@ int orn_cache_create(int device, uint64_t seed, const orn_cache_config* config, 
     const size_t pbytes = (size_t)orn::kWeightCount * 4;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc(&c->params, pbytes) != cudaSuccess || cudaMalloc(&c->m, pbytes) != cudaSuccess ||
-        cudaMalloc(&c->v, pbytes) != cudaSuccess || cudaMalloc(&c->grads, pbytes) != cudaSuccess ||
+        cudaMalloc(&c->v, pbytes) != cudaSuccess || cudaMalloc(&c->grads, pbytes + 8) != cudaSuccess ||
         cudaMalloc(&c->w_f16, (size_t)orn::kWeightCount * 2) != cudaSuccess ||
         cudaMalloc(&c->w_bf16, (size_t)orn::kBackwardWeightCount * 2) != cudaSuccess ||
-        cudaMalloc(&c->d_loss, 4) != cudaSuccess || cudaMalloc(&c->d_status, 4) != cudaSuccess)
+        cudaMallocHost(&c->host, pbytes + 8) != cudaSuccess)
         return bail(ORN_ERR_OUT_OF_MEMORY);
+    c->d_loss = c->grads + orn::kWeightCount;
+    c->d_status = (uint32_t*)(c->grads + orn::kWeightCount + 1);
     // He-uniform weights: U(-sqrt(6 / fan_in), +sqrt(6 / fan_in)); padded
     // output rows zero.
     std::vector<float> w(orn::kWeightCount, 0.0f);
@@ -342,16 +351,10 @@ static int gradients_or_train(orn_cache* c, const float* inputs, const float* ta
     RC_CUDA(c, cudaMemcpyAsync(c->io_target, targets, n * orn::kOutputs * 4, cudaMemcpyHostToDevice, c->stream));
     st = orn::cache_train_step(c, c->io_in, c->io_target, (uint32_t)n, adam, c->d_status, c->stream);
     if (st) return st;
-    if (grads) {
-        RC_CUDA(c, cudaMemcpyAsync(grads, c->grads, (size_t)orn::kWeightCount * 4, cudaMemcpyDeviceToHost,
-                                   c->stream));
-        RC_CUDA(c, cudaMemsetAsync(c->grads, 0, (size_t)orn::kWeightCount * 4, c->stream));
-    }
-    float l = 0.0f;
-    RC_CUDA(c, cudaMemcpyAsync(&l, c->d_loss, 4, cudaMemcpyDeviceToHost, c->stream));
-    st = finish(c);
+    st = finish(c, grads != nullptr);
     if (st) return st;
-    if (loss) *loss = l;
+    if (grads) std::memcpy(grads, c->host, (size_t)orn::kWeightCount * 4);
+    if (loss) *loss = c->host[orn::kWeightCount];
     return ORN_OK;
 }
 

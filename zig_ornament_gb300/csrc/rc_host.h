@@ -26,8 +26,9 @@ struct orn_cache {
     float* grads = nullptr;
     uint16_t* w_f16 = nullptr;
     uint16_t* w_bf16 = nullptr;
-    float* d_loss = nullptr;
-    uint32_t* d_status = nullptr;
+    float* d_loss = nullptr;         // behind the gradients, so that one copy reads all three
+    uint32_t* d_status = nullptr;    // behind the loss
+    float* host = nullptr;           // pinned copy of the gradients, the loss and the status
 
     // per-sample training activations, grown on demand
     uint32_t cap = 0;

@@ -18,13 +18,15 @@ constexpr int kOutPad = 16;                          // output rows padded to th
 constexpr uint32_t kWeightCount = kFeatures * kHidden + 4 * kHidden * kHidden + kHidden * kOutPad;   // 33,792
 constexpr uint32_t kBackwardWeightCount = 4 * kHidden * kHidden + kHidden * kOutPad;                  // layers 2..6
 constexpr uint32_t kTmemCols = 64;
+constexpr int kWgradPerSm = 4;                       // resident weight-gradient CTAs per SM
 constexpr int kWgradJobs = 7;                        // layer 1 in two 128-input blocks + layers 2..6
 constexpr float kGradClamp = 1.0e4f;
 
 // Forward pass over n samples.  Inference writes `outputs` (n x 3) or, when
 // `pixel` is set, adds throughput x max(output, 0) to acc[pixel[i]].xyz;
 // training stores the hidden activations (FP16, [5][n][64]) and the loss
-// gradient of the output (BF16, [n][16]) and sums the loss into *loss.
+// gradient of the output (BF16, [n][16]), sums the loss into *loss and goes
+// back through layers 6..2: dZ(l-1) = (dZ(l) · W(l)) ⊙ [H(l-1) > 0].
 // `n_dev`, when set, supplies n from device memory (a queue length).
 struct RcForward {
     const uint16_t* weights_f16;    // forward operand copies, K-major per layer
@@ -35,19 +37,11 @@ struct RcForward {
     const float4* throughput;       // path throughput per query
     float4* acc;                    // per-pixel accumulation the queries add to
     uint16_t* h_out;                // training: hidden activations
-    uint16_t* dz_out;               // training: output gradients
+    const uint16_t* weights_bf16;   // training: backward operand copies (W(l) with K = outputs)
+    uint16_t* dz6;                  // training: output gradients, [n][16]
+    uint16_t* dz;                   // training: [5][n][64] BF16
     float* loss;
     const uint32_t* n_dev;
-    uint32_t n;
-    uint32_t* status;
-};
-
-// Backward pass through layers 6..2: dZ(l-1) = (dZ(l) · W(l)) ⊙ [H(l-1) > 0].
-struct RcBackward {
-    const uint16_t* weights_bf16;   // backward operand copies (W(l) with K = outputs)
-    const uint16_t* dz6;            // [n][16]
-    const uint16_t* h;              // [5][n][64] FP16
-    uint16_t* dz;                   // [5][n][64] BF16 out
     uint32_t n;
     uint32_t* status;
 };
@@ -85,7 +79,6 @@ __host__ __device__ constexpr uint32_t rc_layer_offset(int l) {
 }
 
 cudaError_t rc_launch_forward(const RcForward& p, bool train, int grid, cudaStream_t s);
-cudaError_t rc_launch_backward(const RcBackward& p, int grid, cudaStream_t s);
 cudaError_t rc_launch_wgrad(const RcWgrad& p, cudaStream_t s);
 cudaError_t rc_launch_adam(const RcAdam& p, cudaStream_t s);
 
