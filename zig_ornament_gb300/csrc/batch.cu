@@ -39,9 +39,13 @@ namespace {
 
 enum BatchLane { B_IDLE = 0, B_TRAVERSE = 1, B_SHADE = 2, B_DONE = 3, B_START = 4 };
 
+// Steps that a lane on the near-first trees makes per pass of its loop (8: 48.2
+// ms for six views, 12: 50.1).
+constexpr int kBatchNearSteps = 8;
+
 // Resident blocks per SM each block size is compiled for: 80 registers a
 // thread at 128 and 192; on the near-first trees, whose step spills 150 bytes
-// there, 96 or more (six scenes, 128 threads: 6 blocks 58.8 ms, 5 52.6).
+// there, 96 or more (six views, 128 threads: 5 blocks 48.1 ms, 6 52.3, 7 53.4).
 template <int BLOCK, bool NEAR> constexpr int batch_min_blocks() {
     return BLOCK == 64 ? 8 : (BLOCK == 128 ? (NEAR ? 5 : 6) : (NEAR ? 3 : 4));
 }
@@ -51,11 +55,10 @@ template <int SEM, bool FAST, bool NEAR, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, batch_min_blocks<BLOCK, NEAR>())
 batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t total_pixels, uint32_t* work_counter,
              uint32_t* error, int shade_threshold) {
-    __shared__ uint32_t sstack[kSmemStack * BLOCK];
+    __shared__ __align__(8) uint32_t sstack[kSmemStack * BLOCK];
     const BatchView* __restrict__ sv = views;
-    TravStack<kSmemStack, NEAR ? kNearStackWords : kStackSize> stack;
-    stack.sstack = sstack + threadIdx.x;
-    stack.sstride = BLOCK;
+    std::conditional_t<NEAR, NearStack<kSmemStack>, TravStack<kSmemStack>> stack;
+    stack.init(sstack, threadIdx.x, BLOCK);
     const unsigned kFull = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lanes_below = (1u << lane) - 1u;
@@ -152,7 +155,7 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
             const float t_min = sv[sc].cp.ray_cast_epsilon;
             if constexpr (NEAR) {
 #pragma unroll 1
-                for (int s = 0; s < kNearSteps; ++s) {
+                for (int s = 0; s < kBatchNearSteps; ++s) {
                     if (!near_step(w, tsc, ro, rd, t_min, stack)) {
                         mode = B_SHADE;
                         break;

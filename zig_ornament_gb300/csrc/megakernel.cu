@@ -85,10 +85,9 @@ template <int SEM, int MATH, bool COUNT, bool FAST, bool F64 = false, bool CACHE
 __global__ void __launch_bounds__(kMegaBlock, CACHE ? ORN_CACHE_MIN_BLOCKS : (NEAR ? kNearMinBlocks : kMegaMinBlocks))
 mega_kernel(RenderLaunch p) {
     static_assert(!NEAR || (FAST && !COUNT && !CACHE), "near-first trees: the plain kernel with the FMNMX slab test");
-    __shared__ uint32_t sstack[kSmemStack * kMegaBlock];
-    TravStack<kSmemStack, NEAR ? kNearStackWords : kStackSize> stack;
-    stack.sstack = sstack + threadIdx.x;
-    stack.sstride = kMegaBlock;
+    __shared__ __align__(8) uint32_t sstack[kSmemStack * kMegaBlock];
+    std::conditional_t<NEAR, NearStack<kSmemStack>, TravStack<kSmemStack>> stack;
+    stack.init(sstack, threadIdx.x, kMegaBlock);
     const unsigned kFull = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lanes_below = (1u << lane) - 1u;
@@ -607,13 +606,12 @@ trace_rays_kernel(SceneDev sc, float t_min, const float* __restrict__ rays, size
 // scene: 920 us).  Rays that the FMNMX slab test does not take are left to
 // trace_rays_kernel: `list`, as there.  (1M rays with their copies 4.4 -> 2.1
 // ms; gathering 4 or 16 idle lanes, 2 or 8 steps between: within 3 %.)
-__global__ void __launch_bounds__(kMegaBlock, kNearMinBlocks)
+__global__ void __launch_bounds__(kMegaBlock, kMegaMinBlocks)
 trace_near_kernel(SceneDev sc, float t_min, const float* __restrict__ rays, uint32_t count,
                   orn_hit* __restrict__ hits, uint32_t* work_counter, uint32_t* list, uint32_t lanes) {
-    __shared__ uint32_t sstack[kSmemStack * kMegaBlock];
+    __shared__ __align__(8) uint32_t sstack[kSmemStack * kMegaBlock];
     NearStack<kSmemStack> stack;
-    stack.sstack = sstack + threadIdx.x;
-    stack.sstride = kMegaBlock;
+    stack.init(sstack, threadIdx.x, kMegaBlock);
     const unsigned kFull = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned mine = lanes == 32u ? kFull : (1u << lanes) - 1u;   // lanes that take rays

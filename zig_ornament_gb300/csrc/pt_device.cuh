@@ -302,28 +302,23 @@ struct VisitCount {
 // Traversal stack: the first SS entries live in shared memory (entry i of
 // this thread at sstack[i * sstride], so a warp's accesses hit 32 distinct
 // banks), deeper entries spill to a per-thread local array; the total size
-// is the reference's 64 entries unless SIZE says otherwise.
-template <int SS, int SIZE = kStackSize>
+// is the reference's 64 entries.
+template <int SS>
 struct TravStack {
     uint32_t* sstack;
     int sstride;
-    uint32_t lstack[SIZE - SS > 0 ? SIZE - SS : 1];
+    uint32_t lstack[kStackSize - SS > 0 ? kStackSize - SS : 1];
+    // `base`: SS * stride words that `stride` threads share
+    __device__ __forceinline__ void init(uint32_t* base, uint32_t thread, int stride) {
+        sstack = base + thread;
+        sstride = stride;
+    }
     __device__ __forceinline__ void put(int i, uint32_t v) {
-        if (SS >= SIZE || i < SS) sstack[i * sstride] = v;
+        if (SS >= kStackSize || i < SS) sstack[i * sstride] = v;
         else lstack[i - SS] = v;
     }
-    // a pair of words at an even place (SS is even)
-    __device__ __forceinline__ void put2(int i, uint32_t a, uint32_t b) {
-        if (SS >= SIZE || i < SS) {
-            sstack[i * sstride] = a;
-            sstack[(i + 1) * sstride] = b;
-        } else {
-            lstack[i - SS] = a;
-            lstack[i + 1 - SS] = b;
-        }
-    }
     __device__ __forceinline__ uint32_t get(int i) const {
-        if (SS >= SIZE || i < SS) return sstack[i * sstride];
+        if (SS >= kStackSize || i < SS) return sstack[i * sstride];
         return lstack[i - SS];
     }
 };

@@ -31,20 +31,26 @@ constexpr int kSmemStack = ORN_SMEM_STACK;
 #endif
 constexpr int kMegaMinBlocks = ORN_MEGA_MIN_BLOCKS;
 
-// The same for the kernel on the near-first trees, and the node visits that a
-// lane makes per pass of its loop.
+// The same for the kernel on the near-first trees, and the steps that a lane
+// makes per pass of its loop.  5, 6 and 7 blocks (ms): 1080p instanced scenes of
+// 16 spp 76.3, 73.2, 71.1 and 73.3, 70.7, 68.1; 1279x719 large scenes 30.7,
+// 32.3, 33.9 and 33.0, 31.7, 32.1; sphere field 10.9, 11.9, 11.5.  More warps
+// against more spills: which of them wins depends on the scene, with up to 9 %
+// to lose.  8 and 12 steps: within 1 % but for small scenes (17.6, 17.2).
 #ifndef ORN_NEAR_MIN_BLOCKS
 #define ORN_NEAR_MIN_BLOCKS 5
 #endif
 constexpr int kNearMinBlocks = ORN_NEAR_MIN_BLOCKS;
 #ifndef ORN_NEAR_STEPS
-#define ORN_NEAR_STEPS 8
+#define ORN_NEAR_STEPS 12
 #endif
 constexpr int kNearSteps = ORN_NEAR_STEPS;
 
 // Node visits of near_step (pt_near.cuh) between looks at triangles and shapes.
+// 4 and 5 of them (ms): instanced scene 76.2, 76.2, large scene 32.9, 33.1,
+// closed room 23.7, 21.4, spheres 9.9, 9.0, six batched views 50.0, 48.8.
 #ifndef ORN_NEAR_INNER
-#define ORN_NEAR_INNER 4
+#define ORN_NEAR_INNER 5
 #endif
 constexpr int kNearInner = ORN_NEAR_INNER;
 

@@ -40,7 +40,6 @@
 
 #include "pt_device.cuh"
 #include "pt_kernels.h"
-#include "pt_kernels.h"
 
 namespace orn {
 
@@ -52,7 +51,7 @@ constexpr uint32_t kNearLeave = 0xffffffffu;  // NearWalker::node: nothing is le
 struct NearWalker {
     uint32_t node;             // next node (typed reference), or kNearLeave
     float near;                // entry of its box
-    int sp, floor;             // words on the stack; those that are not of this space
+    int sp, floor;             // entries on the stack; those that are not of this space
     f3 o, d, inv, oxinv;       // (of the TLAS only while inner nodes of it are visited)
     float t, tie;              // best hit; T of the comment above
     float lim, margin;         // boxes entered beyond `lim` are skipped; the origin's share of the margin
@@ -65,8 +64,29 @@ struct NearWalker {
     bool away;                 // back in the TLAS with the space of a mesh
 };
 
+// The stack of nodes to visit, each with the entry of its box: the first SS / 2
+// in shared memory (as TravStack, 8 bytes an access), the rest in local memory.
 template <int SS>
-using NearStack = TravStack<SS, kNearStackWords>;
+struct NearStack {
+    static_assert(SS % 2 == 0 && SS / 2 < kNearStackSize, "near stack");
+    uint2* sstack;
+    int sstride;
+    uint2 lstack[kNearStackSize - SS / 2];
+    // `base` (8-byte aligned): SS * stride words that `stride` threads share
+    __device__ __forceinline__ void init(uint32_t* base, uint32_t thread, int stride) {
+        sstack = reinterpret_cast<uint2*>(base) + thread;
+        sstride = stride;
+    }
+    __device__ __forceinline__ void put(int i, uint32_t node, float near) {
+        const uint2 v = make_uint2(node, __float_as_uint(near));
+        if (i < SS / 2) sstack[i * sstride] = v;
+        else lstack[i - SS / 2] = v;
+    }
+    __device__ __forceinline__ uint2 get(int i) const {
+        if (i < SS / 2) return sstack[i * sstride];
+        return lstack[i - SS / 2];
+    }
+};
 
 // Moves the ray into a space.
 __device__ __forceinline__ void near_space(NearWalker& w, f3 o, f3 d) {
@@ -94,6 +114,9 @@ __device__ __forceinline__ void walker_begin(NearWalker& w, const SceneDev& sc, 
 }
 
 // aabb_hit_fast that also gives the entry.
+// (mul.rn.f32x2 and add.rn.f32x2 are no way to do two at a time: the compiler
+// makes one fma of them, and a box that the reference misses by a rounding is
+// hit.  Products alone in pairs: no gain.)
 __device__ __forceinline__ bool near_box(float4 mn, float4 mx, f3 inv, f3 oxinv, float t_min, float t_max,
                                          float* entry) {
     const float fx = mx.x * inv.x + oxinv.x, fy = mx.y * inv.y + oxinv.y, fz = mx.z * inv.z + oxinv.z;
@@ -127,11 +150,11 @@ __device__ __forceinline__ void near_pop(NearWalker& w, NearStack<SS>& stack) {
             w.node = kNearLeave;
             return;
         }
-        w.sp -= 2;
-        w.near = __uint_as_float(stack.get(w.sp + 1));
-        if (w.near <= w.lim) break;
+        const uint2 top = stack.get(--w.sp);
+        w.node = top.x;
+        w.near = __uint_as_float(top.y);
+        if (w.near <= w.lim) return;
     }
-    w.node = stack.get(w.sp);
 }
 
 // Tests the two boxes of the lane's inner node and goes on with the nearer.
@@ -145,8 +168,7 @@ __device__ __forceinline__ void near_inner(NearWalker& w, const SceneDev& sc, fl
     const uint32_t lref = bits(nd.a.w), rref = bits(nd.b.w);
     const bool right = hr && (!hl || nr < nl || w.redo);
     if (hl && hr) {
-        stack.put2(w.sp, right ? lref : rref, __float_as_uint(w.redo ? -INFINITY : (right ? nl : nr)));
-        w.sp += 2;
+        stack.put(w.sp++, right ? lref : rref, w.redo ? -INFINITY : (right ? nl : nr));
     }
     if (hl || hr) {
         w.node = right ? rref : lref;

@@ -30,9 +30,9 @@ enum { MATH_PORTABLE = 0, MATH_DEVICE = 1 };  // transcendental implementation
 // ERR_MMA: a tensor-core wait timed out; ERR_WAIT: a wavefront queue wait timed out
 enum { ERR_STACK = 1u, ERR_VISITS = 2u, ERR_MMA = 4u, ERR_WAIT = 8u };
 constexpr uint32_t kRefIndexMask = 0x3FFFFFFFu;
-// Stack of the near-first traversal in words (two per entry; pt_near.cuh), and
-// the mark on a triangle id whose leaf box in its trees is not its own.
-constexpr int kNearStackWords = 128;
+// Entries of the near-first traversal's stack (pt_near.cuh), and the mark on a
+// triangle id whose leaf box in its trees is not its own.
+constexpr int kNearStackSize = 64;
 constexpr uint32_t kNearOwnBox = 0x80000000u;
 
 struct TexDesc {

@@ -48,7 +48,7 @@ constexpr uint32_t kRoundsPerSync = 4;
 constexpr uint32_t kOwnBoxMark = 0x80000000u;   // a leaf's box is not its triangle's own
 constexpr uint32_t kMostSlivers = 64;
 constexpr float kSliver = 1024.0f;
-constexpr uint32_t kNearDepthLimit = kNearStackWords / 2;   // levels of TLAS and BLAS together (one entry of two words each)
+constexpr uint32_t kNearDepthLimit = kNearStackSize;   // levels of TLAS and BLAS together (one entry each)
 
 // Counters and flags of one build (device; read back between phases).
 struct State {

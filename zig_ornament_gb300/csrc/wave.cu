@@ -215,7 +215,7 @@ wave_kernel(RenderLaunch p) {
     if (warp >= (uint32_t)NS) {
         // traversal warps: their lanes' stacks are the first 32 * (NW - NS)
         // columns of the shared stack array
-        traversal_warp<COUNT, FAST, NEAR, P, STEPS>(pool, p, sstack + (threadIdx.x - 32 * NS), 32 * (NW - NS), lane, vc,
+        traversal_warp<COUNT, FAST, NEAR, P, STEPS>(pool, p, sstack, threadIdx.x - 32 * NS, 32 * (NW - NS), lane, vc,
                                               err);
     } else {
         // the shading warp: up to 32 queued hits per round

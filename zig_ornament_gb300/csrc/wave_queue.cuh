@@ -246,12 +246,11 @@ __device__ __forceinline__ void wave_warp(Pool& pool, const RenderLaunch& p, uin
 // the traversal-only role on the 1080p workload).  Returns when the block is
 // finished or a wait ran out.
 template <bool COUNT, bool FAST, bool NEAR, int P, int STEPS, class Pool>
-__device__ __forceinline__ void traversal_warp(Pool& pool, const RenderLaunch& p, uint32_t* sstack, int stride,
-                                               uint32_t lane, VisitCount& vc, uint32_t& err) {
+__device__ __forceinline__ void traversal_warp(Pool& pool, const RenderLaunch& p, uint32_t* sstack, uint32_t thread,
+                                               int stride, uint32_t lane, VisitCount& vc, uint32_t& err) {
     const unsigned kFull = 0xffffffffu;
-    TravStack<kSmemStack, NEAR ? kNearStackWords : kStackSize> stack;
-    stack.sstack = sstack;
-    stack.sstride = stride;
+    std::conditional_t<NEAR, NearStack<kSmemStack>, TravStack<kSmemStack>> stack;
+    stack.init(sstack, thread, stride);
     const float t_min = p.cp.ray_cast_epsilon;
     const int fetch = p.wave_fetch;
     uint32_t slot = kEmpty, steps = 0;
