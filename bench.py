@@ -328,8 +328,8 @@ def profile_figures(name):
 
 # The sources of the megakernel and its launcher (profile figures lines).
 MEGA_SOURCES = ["zig_ornament_gb300/csrc/" + f for f in (
-    "megakernel.cu", "pt_device.cuh", "pt_machine.cuh", "pt_kernels.h", "pt_scene.h", "pmath.h", "qmc.cuh",
-    "capi.cu", "order.cu")] + ["include/ornament_cuda.h", "zig_ornament_gb300/build.py"]
+    "megakernel.cu", "pt_device.cuh", "pt_machine.cuh", "pt_near.cuh", "pt_kernels.h", "pt_scene.h", "pmath.h", "qmc.cuh",
+    "tree_build.cu", "capi.cu", "order.cu")] + ["include/ornament_cuda.h", "zig_ornament_gb300/build.py"]
 
 
 def l1_peak_gbs(clocks, device=0):
@@ -353,7 +353,12 @@ def roofline_block(bytes_per_launch, avg_launch_s, workload, clocks, profile_nam
     latency: `achieved` is the DRAM traffic of one launch over the launch
     time, against the measured HBM copy bandwidth.  `traffic` = DRAM bytes
     per node visit of the ncu capture of this build (a smaller launch of the
-    same scene) x this launch's node visits."""
+    same scene) x this launch's node visits.
+
+    Visits and bytes are those of a counting render, which walks the
+    reference's trees.  The timed kernel's near-first trees need about half
+    the visits, so `achieved` is a rate of the reference's work, and DRAM
+    bytes per visit are per visit of the reference's walk."""
     peak_hbm, kind = measured_peaks()
     algo = bytes_per_launch / avg_launch_s / 1e9
     fig, src = profile_figures(profile_name) if profile_name else (None, "no profile")

@@ -245,7 +245,11 @@ typedef struct orn_context orn_context;
 /* PathTracer.init — src/hip_backend/path_tracer.zig:36-86.  Copies every
  * blob array to device `device` (-1 = the last device, as the HIP backend
  * picks, src/hip_backend/path_tracer.zig:40).  The caller keeps ownership
- * of the blob.  Validates every index in the blob. */
+ * of the blob.  Validates every index in the blob.  Where the blob's boxes
+ * contain what is below them and the trees have at most 64 levels, a second
+ * set of trees over the same primitives is built beside the blob's (as much
+ * memory again as its nodes), which plain renders and ray queries walk nearest
+ * box first; the hits are those of the blob's trees. */
 int orn_create(const orn_scene_blob* blob, int device, orn_context** out);
 
 /* PathTracer.deinit — src/hip_backend/path_tracer.zig:88-101. */
@@ -326,7 +330,8 @@ int orn_peek_constant_params(const orn_context* ctx, orn_constant_params* out);
 
 /* Bvh::hit on a list of rays — src/hip_backend/kernels/bvh.hip.h:145-276.
  * Writes one orn_hit per ray and, if `visits` is not NULL, the number of
- * traversal-loop iterations (node visits) each ray took.  Synchronous. */
+ * traversal-loop iterations (node visits) each ray took in the blob's trees
+ * (counting them is slower: the rays walk those).  Synchronous. */
 int orn_trace_rays(orn_context* ctx, const orn_ray* rays, size_t count,
                    orn_hit* hits, uint32_t* visits);
 

@@ -164,3 +164,27 @@ def test_blobs_with_other_boxes_keep_the_reference_walk():
         got, _ = r.trace_rays(rays, with_visits=False)
         r.close()
         assert np.array_equal(want.view(np.uint32), got.view(np.uint32))
+
+
+@pytest.mark.parametrize("builder", ["reference", "sah", "lbvh"])
+@pytest.mark.parametrize("semantics", [_lib.SEMANTICS_HIP, _lib.SEMANTICS_WGSL], ids=["hip", "wgsl"])
+def test_large_scenes_render_the_same_on_any_tree_rule(builder, semantics):
+    """Past 16384 nodes the trees' areas decide what a plain render walks; a
+    counting render always walks the blob's."""
+    w, h = 97, 53
+    scene = scenes.instanced_meshes_scene(w, h, seed=3, n_blas=2, n_instances=24, tri_range=(8_000, 12_000),
+                                          texture_size=32)
+    bvh = ornament.Bvh(scene, builder=builder)
+    frames = []
+    for count in (False, True):
+        pt = ornament.PathTracer(scene, bvh=bvh)
+        scene.camera.dirty = True
+        pt.state.setDepth(8)
+        pt.state.setIterations(3)
+        pt.state.semantics = semantics
+        pt.setResolution(ornament.Resolution(w, h))
+        pt.renderer.enable_counters(count)
+        pt.render()
+        frames.append(pt.getFrameBuffer().copy())
+        pt.deinit()
+    assert np.array_equal(frames[0].view(np.uint32), frames[1].view(np.uint32))

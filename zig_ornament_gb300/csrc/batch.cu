@@ -113,10 +113,7 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
     };
 
     for (;;) {
-        for (;;) {   // (one copy of start_samples, as in the megakernel)
-            if (mode == B_START) mode = start_samples();
-            const unsigned idle = __ballot_sync(kFull, mode == B_IDLE);
-            if (idle == 0u || exhausted) break;
+        auto hand_out = [&](unsigned idle) {
             const unsigned leader = __ffs(idle) - 1u;
             const unsigned n = __popc(idle);
             uint32_t base = 0;
@@ -142,9 +139,20 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
                     rng.state = sv[sc].rng[gid];
                     acc = sv[sc].cp.current_iteration > 1.0f ? sv[sc].acc[gid] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     k = 0;
-                    mode = B_START;
+                    mode = NEAR ? (int)B_START : start_samples();
                 }
             }
+        };
+        if constexpr (NEAR) {
+            for (;;) {   // (one copy of start_samples, as in the megakernel)
+                if (mode == B_START) mode = start_samples();
+                const unsigned idle = __ballot_sync(kFull, mode == B_IDLE);
+                if (idle == 0u || exhausted) break;
+                hand_out(idle);
+            }
+        } else {
+            const unsigned idle = __ballot_sync(kFull, mode == B_IDLE);
+            if (idle != 0u && !exhausted) hand_out(idle);
         }
         if (exhausted && mode == B_IDLE) mode = B_DONE;
         if (__ballot_sync(kFull, mode == B_TRAVERSE || mode == B_SHADE) == 0u &&
@@ -185,7 +193,7 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
                     else color = sky_color(color, rd);
                     cont = false;
                 } else {
-                    cont = shade_hit<SEM, MATH_PORTABLE, false>(V.scene, V.cp, rng, h, &ro, &rd, &color, &scn);
+                    cont = shade_hit<SEM, MATH_PORTABLE, false, !NEAR>(V.scene, V.cp, rng, h, &ro, &rd, &color, &scn);
                 }
                 if (cont && ++bounce < V.cp.depth) {
                     walker_begin(w, tsc, ro, rd);
@@ -193,7 +201,7 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
                 } else {
                     add_sample(V.cp.current_iteration + (float)k);
                     ++k;
-                    mode = B_START;
+                    mode = NEAR ? (int)B_START : start_samples();
                 }
             }
         }
@@ -341,7 +349,7 @@ int prepare_frame(orn_batch* b, uint32_t* total_pixels, uint32_t* semantics, int
         v.pixel_begin = (uint32_t)total;
         total += (uint64_t)v.cp.width * v.cp.height;
         if (total >= 0xFFFFFFFFull) return bfail(b, ORN_ERR_INVALID_ARGUMENT, "batch frame too large");
-        all = std::min<int>(all, !f ? orn::BATCH_EXACT : (v.scene.near ? orn::BATCH_NEAR : orn::BATCH_FAST));
+        all = std::min<int>(all, !f ? orn::BATCH_EXACT : (v.scene.near > 1u ? orn::BATCH_NEAR : orn::BATCH_FAST));
         b->h_views[i] = v;
     }
     *total_pixels = (uint32_t)total;
@@ -545,7 +553,7 @@ int orn_batch_tune(orn_batch* b, const char* cache_path, orn_batch_config* chose
         int dev = 0;
         int st = orn::batch_prepare(b->contexts[i], &saved[i], &f, &sm, &dev, b->stream, false);
         if (st) return bfail(b, st, orn_last_error(b->contexts[i]));
-        slabs = std::min<int>(slabs, !f ? orn::BATCH_EXACT : (saved[i].scene.near ? orn::BATCH_NEAR : orn::BATCH_FAST));
+        slabs = std::min<int>(slabs, !f ? orn::BATCH_EXACT : (saved[i].scene.near > 1u ? orn::BATCH_NEAR : orn::BATCH_FAST));
         sem = sm;
         const uint32_t px = saved[i].cp.width * saved[i].cp.height;
         saved[i].pixel_begin = (uint32_t)total64;

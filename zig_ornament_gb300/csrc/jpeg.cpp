@@ -1,7 +1,7 @@
 // jpeg.cpp — JPEG (ITU-T T.81) sequential Huffman decoding on the host: the
-// marker parser and the entropy decoder, which produce one plane of
-// quantised DCT coefficients per component.  The arithmetic stages run on
-// the GPU (jpeg.cu).
+// marker parser and the entropy decoder, which produce the nonzero quantised
+// DCT coefficients of every block.  The arithmetic stages run on the GPU
+// (jpeg.cu).
 //
 // Handled: SOF0 / SOF1 (8-bit samples), 1 or 3 components with sampling
 // factors 1..4, interleaved and non-interleaved scans (several scans per
@@ -13,7 +13,8 @@
 // the input buffer.
 //
 // Procedures follow the standard: Huffman tables from BITS/HUFFVAL (Annex C),
-// DECODE with MAXCODE/VALPTR (F.2.2.3, here behind a 9-bit lookup),
+// DECODE with MAXCODE/VALPTR (F.2.2.3, here behind a table of the next 11
+// bits that also holds short codes' values),
 // RECEIVE/EXTEND (F.2.2.1), the zig-zag sequence (Figure A.6), MCU order
 // (A.2).
 #include <algorithm>

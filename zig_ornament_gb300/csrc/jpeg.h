@@ -1,6 +1,6 @@
 // jpeg.h — sequential (baseline / extended Huffman) JPEG parsing and entropy
 // decoding on the host (jpeg.cpp); the GPU stage (jpeg.cu) dequantises,
-// inverse-transforms, upsamples and colour-converts the coefficient planes.
+// inverse-transforms, upsamples and colour-converts the coefficients.
 //
 // This is the texture path of the reference's example app: textures are
 // loaded with zstbi (stb_image) as 4-component images, flipped vertically

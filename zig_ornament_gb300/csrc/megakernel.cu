@@ -81,7 +81,7 @@ template <> struct Accum<true> {
 #define ORN_CACHE_MIN_BLOCKS 7
 #endif
 template <int SEM, int MATH, bool COUNT, bool FAST, bool F64 = false, bool CACHE = false, bool SOBOL = false,
-          bool NEAR = false>
+          bool NEAR = false, bool SPLIT = !NEAR && !CACHE>
 __global__ void __launch_bounds__(kMegaBlock, CACHE ? ORN_CACHE_MIN_BLOCKS : (NEAR ? kNearMinBlocks : kMegaMinBlocks))
 mega_kernel(RenderLaunch p) {
     static_assert(!NEAR || (FAST && !COUNT && !CACHE), "near-first trees: the plain kernel with the FMNMX slab test");
@@ -190,14 +190,8 @@ mega_kernel(RenderLaunch p) {
     };
 
     for (;;) {
-        // Lanes whose sample is complete start the next one (or complete the
-        // pixel), and idle lanes are handed pixels, one atomic per warp, until
-        // every lane has a ray or the pixels run out.  (start_samples is long:
-        // one copy of it, for the instruction cache.)
-        for (;;) {
-            if (mode == LANE_START) mode = start_samples();
-            const unsigned idle = __ballot_sync(kFull, mode == LANE_IDLE);
-            if (idle == 0u || exhausted) break;
+        // Idle lanes are handed pixels, one atomic per warp.
+        auto hand_out = [&](unsigned idle) {
             const unsigned leader = __ffs(idle) - 1u;
             const unsigned n = __popc(idle);
             uint32_t base = 0;
@@ -222,9 +216,24 @@ mega_kernel(RenderLaunch p) {
                         rng.state = p.rng[gid];
                         acc.load(p, gid, ci0);
                     }
-                    mode = LANE_START;
+                    mode = SPLIT ? start_samples() : (int)LANE_START;
                 }
             }
+        };
+        if constexpr (!SPLIT) {
+            // Lanes whose sample is complete start the next one (or complete
+            // the pixel), until every lane has a ray or the pixels run out:
+            // one copy of start_samples, which is long, for the instruction
+            // cache.  (SPLIT: see SplitGeom.)
+            for (;;) {
+                if (mode == LANE_START) mode = start_samples();
+                const unsigned idle = __ballot_sync(kFull, mode == LANE_IDLE);
+                if (idle == 0u || exhausted) break;
+                hand_out(idle);
+            }
+        } else {
+            const unsigned idle = __ballot_sync(kFull, mode == LANE_IDLE);
+            if (idle != 0u && !exhausted) hand_out(idle);
         }
         if (exhausted && mode == LANE_IDLE) mode = LANE_DONE;
         if (__ballot_sync(kFull, mode == LANE_TRAVERSE || mode == LANE_SHADE) == 0u &&
@@ -298,7 +307,7 @@ mega_kernel(RenderLaunch p) {
                         const float4 ma = ldg4(p.scene.materials + 2 * (size_t)h.material);
                         const float4 mb = ldg4(p.scene.materials + 2 * (size_t)h.material + 1);
                         const uint32_t mtype = bits(mb.z);
-                        const HitGeom g = hit_geometry<MATH, COUNT>(p.scene, h, ro, rd, &scn);
+                        const auto g = geometry<SPLIT, MATH, COUNT>(p.scene, h, ro, rd, &scn);
                         if (mtype > ORN_DIELECTRIC) {
                             // emitter (or unknown type): the path ends with color x emission,
                             // unless the previous vertex sampled this emitter directly
@@ -519,7 +528,7 @@ mega_kernel(RenderLaunch p) {
                         }
                         add_sample(c);
                         ++k;
-                        mode = LANE_START;
+                        mode = SPLIT ? start_samples() : (int)LANE_START;
                     }
                 } else {
                     bool cont, any;
@@ -530,7 +539,7 @@ mega_kernel(RenderLaunch p) {
                         else color = sky_color(color, rd);
                         cont = false;
                     } else {
-                        cont = shade_hit<SEM, MATH, COUNT>(p.scene, p.cp, rng, h, &ro, &rd, &color, &scn);
+                        cont = shade_hit<SEM, MATH, COUNT, SPLIT>(p.scene, p.cp, rng, h, &ro, &rd, &color, &scn);
                     }
                     if (cont && ++bounce < p.cp.depth) {
                         if (COUNT) scn.rays++;
@@ -539,7 +548,7 @@ mega_kernel(RenderLaunch p) {
                     } else {
                         acc.add(ci0 + (float)k, color);
                         ++k;
-                        mode = LANE_START;
+                        mode = SPLIT ? start_samples() : (int)LANE_START;
                     }
                 }
             }
@@ -737,7 +746,7 @@ cudaError_t launch_relmse(const float4* acc, const double* acc64, const double* 
 // Persistent grid: as many blocks as fit on the device at once (never more
 // than the pixels need).
 template <int SEM, int MATH, bool COUNT, bool FAST, bool F64 = false, bool CACHE = false, bool SOBOL = false,
-          bool NEAR = false>
+          bool NEAR = false, bool SPLIT = !NEAR && !CACHE>
 static cudaError_t launch_mega_tt(const RenderLaunch& p, cudaStream_t s) {
     static int blocks_per_sm = 0, sms = 0;
     if (blocks_per_sm == 0) {
@@ -746,10 +755,10 @@ static cudaError_t launch_mega_tt(const RenderLaunch& p, cudaStream_t s) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 #ifdef ORN_MEGA_CARVEOUT
         // shared-memory share of the unified L1/shared space, in percent
-        cudaFuncSetAttribute(mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR>,
+        cudaFuncSetAttribute(mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR, SPLIT>,
                              cudaFuncAttributePreferredSharedMemoryCarveout, ORN_MEGA_CARVEOUT);
 #endif
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR>,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR, SPLIT>,
                                                       kMegaBlock, 0);
         if (blocks_per_sm < 1) blocks_per_sm = 1;
     }
@@ -769,29 +778,31 @@ static cudaError_t launch_mega_tt(const RenderLaunch& p, cudaStream_t s) {
     if (need < grid) grid = need;
     cudaError_t e = cudaMemsetAsync(p.work_counter, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR><<<grid, kMegaBlock, 0, s>>>(q);
+    mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR, SPLIT><<<grid, kMegaBlock, 0, s>>>(q);
     return cudaGetLastError();
 }
 
 // The Sobol sampler is a separate instantiation, so the stream sampler's
 // kernel carries none of its code.
-template <bool SOBOL>
-static cudaError_t launch_mega_cached_t(const RenderLaunch& p, int semantics, bool fast, cudaStream_t s) {
-    if (semantics == SEM_WGSL)
-        return fast ? launch_mega_tt<SEM_WGSL, MATH_PORTABLE, false, true, false, true, SOBOL>(p, s)
-                    : launch_mega_tt<SEM_WGSL, MATH_PORTABLE, false, false, false, true, SOBOL>(p, s);
-    return fast ? launch_mega_tt<SEM_HIP, MATH_PORTABLE, false, true, false, true, SOBOL>(p, s)
-                : launch_mega_tt<SEM_HIP, MATH_PORTABLE, false, false, false, true, SOBOL>(p, s);
+template <int SEM, bool SOBOL>
+static cudaError_t launch_mega_cached_t(const RenderLaunch& p, bool fast, cudaStream_t s) {
+    if (!fast) return launch_mega_tt<SEM, MATH_PORTABLE, false, false, false, true, SOBOL>(p, s);
+    // walking counts for more than shading (SplitGeom)
+    if (p.scene.large) return launch_mega_tt<SEM, MATH_PORTABLE, false, true, false, true, SOBOL, false, true>(p, s);
+    return launch_mega_tt<SEM, MATH_PORTABLE, false, true, false, true, SOBOL>(p, s);
 }
 
 cudaError_t launch_mega_cached(const RenderLaunch& p, int semantics, bool fast, cudaStream_t s) {
-    return p.cache.sobol ? launch_mega_cached_t<true>(p, semantics, fast, s)
-                         : launch_mega_cached_t<false>(p, semantics, fast, s);
+    if (semantics == SEM_WGSL)
+        return p.cache.sobol ? launch_mega_cached_t<SEM_WGSL, true>(p, fast, s)
+                             : launch_mega_cached_t<SEM_WGSL, false>(p, fast, s);
+    return p.cache.sobol ? launch_mega_cached_t<SEM_HIP, true>(p, fast, s)
+                         : launch_mega_cached_t<SEM_HIP, false>(p, fast, s);
 }
 
 template <int SEM>
 static cudaError_t launch_mega_t(const RenderLaunch& p, bool count, bool fast, cudaStream_t s) {
-    if (fast && !count && p.scene.near)
+    if (fast && !count && p.scene.near > 1u)
         return launch_mega_tt<SEM, MATH_PORTABLE, false, true, false, false, false, true>(p, s);
     if (fast) return count ? launch_mega_tt<SEM, MATH_PORTABLE, true, true>(p, s)
                            : launch_mega_tt<SEM, MATH_PORTABLE, false, true>(p, s);
@@ -800,7 +811,7 @@ static cudaError_t launch_mega_t(const RenderLaunch& p, bool count, bool fast, c
 }
 
 cudaError_t launch_mega_f64(const RenderLaunch& p, int semantics, bool fast, cudaStream_t s) {
-    if (fast && p.scene.near)
+    if (fast && p.scene.near > 1u)
         return semantics == SEM_WGSL ? launch_mega_tt<SEM_WGSL, MATH_PORTABLE, false, true, true, false, false, true>(p, s)
                                      : launch_mega_tt<SEM_HIP, MATH_PORTABLE, false, true, true, false, false, true>(p, s);
     if (semantics == SEM_WGSL)

@@ -8,7 +8,9 @@
 //
 // Here every lane holds one path and the warp runs ONE loop whose condition
 // comes from warp ballots, so the lanes stay converged:
-//   * each iteration, every lane in the TRAVERSE state visits one BVH node;
+//   * each iteration, every lane in the TRAVERSE state visits one BVH node
+//     (walker_step), or takes a few steps on the near-first trees
+//     (pt_near.cuh) where the scene has them;
 //   * lanes whose ray finished traversal wait in SHADE until enough of the
 //     warp is ready (or nobody is traversing), then all ready lanes shade
 //     together (material scatter, next bounce, next sample, pixel done);

@@ -58,8 +58,10 @@ struct SceneDev {
     // Other trees over the same primitives (tree_build.cu), for the traversal
     // of pt_near.cuh: behind the nodes above in the same array and format.
     // `near` is 0 when the scene's arrays do not have what its proof of equal
-    // results needs; the nodes above are then walked everywhere.
+    // results needs, and the nodes above are then walked everywhere; 1 when the
+    // nodes above are good trees themselves, which renders walk faster; else 2.
     uint32_t near;
+    uint32_t large;             // enough nodes that walking them outweighs shading
     uint32_t nroot;             // reference of the TLAS root
 };
 

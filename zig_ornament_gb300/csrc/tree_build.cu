@@ -38,6 +38,18 @@ namespace {
 
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr uint32_t kTlasTree = 0x3fffffffu;   // tree id of the TLAS (meshes: their root's BLAS index)
+// Scenes of this many nodes (1 MB, more than an L1) are taken to spend more on
+// walking than on shading: the sphere field (975) and rooms (40) do not, the
+// mesh scenes (563 k and 2 M) do.
+constexpr uint32_t kLargeScene = 16384;
+// A large scene's renders stay on the blob's trees when the boxes of their
+// BLASes have less than this many times the near-first trees' area.  Binned-SAH
+// trees have 0.92, GPU-built linear ones 1.08 to 1.10, the reference's median
+// splits 1.77 to 1.84.  The first two are as good, and the reference's walk
+// costs less per visit (1080p scene of 16 passes, blob's trees against
+// near-first: SAH 65.7 and 76.8 ms, linear 70.1 and 76.9, reference 91.3 and
+// 77.0).  Ray lists, where latency counts, always take the near-first trees.
+constexpr float kGoodTrees = 1.35f;
 constexpr uint32_t kDepthLimit = 64;          // the reference's stack entries
 constexpr int kRadius = 16;
 constexpr int kNnBlock = 256;
@@ -63,7 +75,15 @@ struct State {
     uint32_t clusters;    // left to merge
     uint32_t near_depth[2];   // levels of the deepest BLAS, and of the TLAS
     uint32_t root;        // reference of the TLAS root
+    float area[2];        // of the inner nodes' children's boxes: the blob's BLASes, the new ones
 };
+
+// Adds a warp's half box areas (lanes without one: 0) to *sum.
+__device__ __forceinline__ void add_area(float* sum, float a) {
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if ((threadIdx.x & 31u) == 0u && a != 0.0f) atomicAdd(sum, a);
+}
+__device__ __forceinline__ float half_area(float x, float y, float z) { return x * y + y * z + z * x; }
 
 __device__ __forceinline__ uint32_t ref_of(const orn_bvh_node* nodes, uint32_t i, uint32_t offset) {
     return (offset + i) | (nodes[i].node_type << 30);
@@ -556,6 +576,33 @@ __global__ void roots_kernel(Emit e, const uint32_t* __restrict__ cluster, uint3
     atomicMax(&e.st->near_depth[tree == kTlasTree ? 1 : 0], levels);
 }
 
+// Half areas of the boxes that the blob's BLAS inner nodes hold.
+__global__ void blob_area_kernel(const orn_bvh_node* __restrict__ blas, uint32_t n, float* sum) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    float a = 0.0f;
+    if (i < n && blas[i].node_type == ORN_NODE_INTERNAL)
+        for (int side = 0; side < 2; ++side) {
+            float lo[3], hi[3];
+            stored_box(blas[i], side != 0, lo, hi);
+            a += half_area(hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2]);
+        }
+    add_area(sum, a);
+}
+// The same of the new BLAS nodes: those that are not the TLAS's.
+__global__ void near_area_kernel(Emit e, uint32_t total, float* sum) {
+    const uint32_t c = e.n + blockIdx.x * blockDim.x + threadIdx.x;
+    float a = 0.0f;
+    if (c < total) {
+        const uint2 ch = e.child[c - e.n];
+        for (int side = 0; side < 2; ++side) {
+            const uint32_t k = side ? ch.y : ch.x;
+            const float4 lo = e.node_box[2 * (size_t)k], hi = e.node_box[2 * (size_t)k + 1];
+            if (__float_as_uint(lo.w) != kTlasTree) a += half_area(hi.x - lo.x, hi.y - lo.y, hi.z - lo.z);
+        }
+    }
+    add_area(sum, a);
+}
+
 __global__ void write_kernel(Emit e, uint32_t total) {
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= total) return;
@@ -726,11 +773,15 @@ cudaError_t Build::near_trees(Arena& a) {
     roots_kernel<<<blocks(trees, 128), 128, 0, s>>>(e, cluster, trees);
     write_kernel<<<blocks(total, 256), 256, 0, s>>>(e, total);
     meshes_kernel<<<blocks(T, 128), 128, 0, s>>>(e.out, T, e.root_of, e.mesh_place, d_state);
+    if (scene->large) {
+        if (B) blob_area_kernel<<<blocks(B, 256), 256, 0, s>>>(blas, B, &d_state->area[0]);
+        if (total > n) near_area_kernel<<<blocks(total - n, 256), 256, 0, s>>>(e, total, &d_state->area[1]);
+    }
     WB(cudaGetLastError());
     WB(read_state());
     if (h.near_depth[0] + h.near_depth[1] > kNearDepthLimit) return cudaSuccess;
     scene->nroot = h.root;
-    scene->near = 1u;
+    scene->near = scene->large && h.area[0] < kGoodTrees * h.area[1] ? 1u : 2u;
     return cudaSuccess;
 }
 
@@ -751,6 +802,7 @@ cudaError_t build_scene_trees(const orn_scene_blob* blob, const float4* d_xforms
     b.nodes = (float4*)nodes;
     scene->nodes = b.nodes;
     scene->near = 0u;
+    scene->large = (uint64_t)blob->tlas_nodes_len + blob->blas_nodes_len >= kLargeScene ? 1u : 0u;
     Arena a;
     a.size = first_bytes(T, B);
     WB(cudaMalloc((void**)&a.base, a.size));

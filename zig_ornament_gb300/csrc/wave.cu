@@ -14,7 +14,7 @@
 // (traversal_warp; nine of ten in the default block shape) — idle lanes
 // take the next rays from the ray queue (ballot-compacted, one reservation
 // per warp) once enough of them are idle (p.wave_fetch, default four),
-// each lane visits BVH nodes (walker_step, the megakernel's traversal) and,
+// each lane visits BVH nodes (near_step or walker_step, as the megakernel) and,
 // when its ray is done, writes the hit record into the slot and appends the
 // slot to the hit queue — and one shades: it takes up to 32 slots from the
 // hit queue and runs the path logic with a full warp —
@@ -344,7 +344,7 @@ cudaError_t launch_wave_steps(const RenderLaunch& p, int shape, cudaStream_t s) 
 template <int SEM, bool FAST>
 cudaError_t launch_wave_shape(const RenderLaunch& p, const WaveConfig& c, bool count, cudaStream_t s) {
     if (count) return launch_wave_t<SEM, true, FAST, false, 0, 32>(p, s);
-    if (FAST && p.scene.near)
+    if (FAST && p.scene.near > 1u)
         return c.steps == 64 ? launch_wave_steps<SEM, FAST, FAST, 64>(p, c.shape, s)
                              : launch_wave_steps<SEM, FAST, FAST, 32>(p, c.shape, s);
     return c.steps == 64 ? launch_wave_steps<SEM, FAST, false, 64>(p, c.shape, s)
