@@ -335,6 +335,11 @@ int orn_peek_constant_params(const orn_context* ctx, orn_constant_params* out);
 int orn_trace_rays(orn_context* ctx, const orn_ray* rays, size_t count,
                    orn_hit* hits, uint32_t* visits);
 
+/* Which trees this context's plain renders and ray queries walk (with the
+ * present state; see orn_create): 0 the blob's; 1 renders the blob's, ray
+ * queries without visits the second set; 2 both the second set. */
+int orn_near_trees(const orn_context* ctx, uint32_t* out);
+
 /* Work counters of the last orn_render (zeros unless enabled with
  * orn_enable_counters): [0] samples, [1] extension rays, [2] node visits,
  * [3] internal-node visits, [4] sphere-leaf visits, [5] mesh-entry visits,

@@ -182,6 +182,7 @@ FUNCTIONS = {
     "orn_set_progress": (C.c_int, [_P, _P, _P, C.c_size_t, C.c_float]),
     "orn_peek_constant_params": (C.c_int, [_P, C.POINTER(ConstantParams)]),
     "orn_trace_rays": (C.c_int, [_P, _P, C.c_size_t, _P, _P]),
+    "orn_near_trees": (C.c_int, [_P, C.POINTER(C.c_uint32)]),
     "orn_enable_counters": (C.c_int, [_P, C.c_int]),
     "orn_get_counters": (C.c_int, [_P, C.POINTER(C.c_uint64), C.c_size_t]),
     "orn_last_render_ms": (C.c_int, [_P, C.POINTER(C.c_float)]),

@@ -1092,6 +1092,12 @@ int orn_trace_rays(orn_context* ctx, const orn_ray* rays, size_t count, orn_hit*
     return st;
 }
 
+int orn_near_trees(const orn_context* ctx, uint32_t* out) {
+    if (!ctx || !out) return ORN_ERR_INVALID_ARGUMENT;
+    *out = ctx->scene.exact_slabs ? 0u : ctx->scene.near;
+    return ORN_OK;
+}
+
 int orn_render_f64(orn_context* ctx, uint32_t spp, double* mean_rgba, size_t pixel_count) {
     if (!ctx || !mean_rgba || spp == 0) return ORN_ERR_INVALID_ARGUMENT;
     if (!ctx->camera_set) return fail(ctx, ORN_ERR_INVALID_ARGUMENT, "no camera set (orn_set_camera)");

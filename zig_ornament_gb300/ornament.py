@@ -740,6 +740,13 @@ class Renderer:
                                              _ptr(visits) if with_visits else None))
         return hits, visits
 
+    def near_trees(self) -> int:
+        """0: the blob's trees are walked; 1: ray queries without visits take
+        the near-first trees; 2: plain renders too (orn_near_trees)."""
+        n = C.c_uint32()
+        self._check(self._lib.orn_near_trees(self._ctx, C.byref(n)))
+        return n.value
+
     def enable_counters(self, enable: bool = True):
         self._check(self._lib.orn_enable_counters(self._ctx, 1 if enable else 0))
 
