@@ -4,8 +4,8 @@
 //   1. The blob's nodes go to the device as they are; one pass writes the
 //      kernels' node array (pt_scene.h), a second finds every node's parent
 //      and checks what the near-first traversal's proof of equal results
-//      needs: each stored box holds the boxes stored below it, a triangle's
-//      box is that of its vertices, no node has two parents, and no walk can
+//      needs: each stored box has its lower corner first and holds the boxes
+//      stored below it, a triangle's box is that of its vertices, no node has two parents, and no walk can
 //      need more than the reference's 64 stack entries.  A blob without one
 //      of these (other builders' padding, shared subtrees) keeps the
 //      reference's walk.
@@ -161,6 +161,9 @@ __global__ void parents_kernel(const orn_bvh_node* __restrict__ nodes, uint32_t 
         if (atomicExch(&parent[c], i | (side ? 0x80000000u : 0u)) != kNone) ok = false;
         float lo[3], hi[3];
         stored_box(nd, side != 0, lo, hi);
+        // (a sphere of negative radius has its box the wrong way round: the slab
+        // test takes it as it is, but no box above it holds it)
+        for (int k = 0; k < 3; ++k) ok = ok && lo[k] <= hi[k];
         const orn_bvh_node ch = nodes[c];
         if (ch.node_type == ORN_NODE_INTERNAL) {
             for (int s2 = 0; s2 < 2; ++s2) {
