@@ -3,7 +3,7 @@ walk's: closest hits bit for bit those of the walk that counts visits."""
 import numpy as np
 import pytest
 
-from zig_ornament_gb300 import ornament
+from zig_ornament_gb300 import ornament, scenes
 from zig_ornament_gb300.ornament import F32
 
 pytestmark = pytest.mark.gpu
@@ -52,3 +52,9 @@ def test_negative_radii():
         r = rs.uniform(0.3, 1.2)
         s.createSphere((*rs.uniform(-4, 4, 3), 1), -r if i % 3 == 0 else r, grey)
     _assert_same_hits(s, 5.0, trees=0)
+
+
+@pytest.mark.parametrize("epsilon,trees", [(1.0, 2), (-0.001, 0), (-5.0, 0), (float("nan"), 0)])
+def test_ray_cast_epsilon(epsilon, trees):
+    """The near-first trees are walked for hits from the origin on, not for hits behind it."""
+    _assert_same_hits(scenes.spheres_scene(), 12.0, epsilon, trees)

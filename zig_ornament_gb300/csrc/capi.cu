@@ -40,6 +40,7 @@ struct orn_context {
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
     std::vector<void*> scene_allocs;
     SceneDev scene{};
+    uint32_t near_built = 0;          // SceneDev::near as the trees allow it
     uint32_t scene_textures_count = 0;
     uint32_t tlas_len = 0, blas_len = 0;
     double world_extent = 0.0;        // largest |coordinate| of the TLAS bounds
@@ -131,6 +132,13 @@ int cuda_fail(orn_context* ctx, cudaError_t e, const char* what) {
         cudaError_t e_ = (call);                                    \
         if (e_ != cudaSuccess) return cuda_fail((ctx), e_, #call);  \
     } while (0)
+
+// The near-first trees serve rays that begin at their origin or beyond:
+// behind it a box is entered after it is left, and the order of entries says
+// nothing about t (ray_cast_epsilon < 0 or NaN: the blob's trees are walked).
+void use_near_trees(orn_context* ctx) {
+    ctx->scene.near = ctx->state.ray_cast_epsilon >= 0.0f ? ctx->near_built : 0u;
+}
 
 orn_state default_state() {
     orn_state s;
@@ -751,6 +759,7 @@ int orn_create(const orn_scene_blob* blob, int device, orn_context** out) {
         if ((s = upload(ctx, descs.data(), descs.size(), &d_t))) return s;
         orn::NodeFacts facts{};
         ORN_CUDA(ctx, orn::build_scene_trees(blob, d_x, &ctx->scene, &facts, &ctx->scene_allocs, ctx->stream));
+        ctx->near_built = ctx->scene.near;
         ctx->scene.tlas_len = blob->tlas_nodes_len;
         ctx->scene.node_count = blob->tlas_nodes_len + blob->blas_nodes_len;
         ctx->scene.root_ref = (blob->tlas_nodes_len - 1) |
@@ -853,6 +862,7 @@ int orn_set_state(orn_context* ctx, const orn_state* s) {
         s->sampler > ORN_SAMPLER_SOBOL)
         return fail(ctx, ORN_ERR_INVALID_ARGUMENT, "unknown semantics, kernel or triangle test");
     ctx->state = *s;
+    use_near_trees(ctx);
     ctx->scene.watertight = s->triangle_test == ORN_TRIANGLE_WATERTIGHT ? 1u : 0u;
     return ORN_OK;
 }
