@@ -249,7 +249,10 @@ typedef struct orn_context orn_context;
  * contain what is below them and the trees have at most 64 levels, a second
  * set of trees over the same primitives is built beside the blob's (as much
  * memory again as its nodes), which plain renders and ray queries walk nearest
- * box first; the hits are those of the blob's trees. */
+ * box first (orn_near_trees).  The hits are those of the blob's trees, but
+ * where a ray runs in a triangle's plane, to within rounding: the reference's
+ * test then gives a t that is rounding alone, and which surface such a ray hits
+ * depends on the order of its visits. */
 int orn_create(const orn_scene_blob* blob, int device, orn_context** out);
 
 /* PathTracer.deinit — src/hip_backend/path_tracer.zig:88-101. */

@@ -66,12 +66,12 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
     int mode = B_IDLE;
     bool exhausted = false;
     uint32_t sc = 0, gid = 0, k = 0, bounce = 0;
-    // the lane's scene as traversal sees it: walker_begin and the steps read
-    // only the node array, the roots and the triangle-test choice
+    // the lane's scene as traversal sees it: the steps, and walker_begin but for
+    // the near-first trees, read only the node array, the root and the
+    // triangle-test choice
     SceneDev tsc;
     tsc.nodes = nullptr;
     tsc.root_ref = 0;
-    tsc.nroot = 0;
     tsc.exact_slabs = 0;
     tsc.watertight = 0;
     Rng rng{0};
@@ -84,6 +84,10 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
     SampleCount scn = {0, 0, 0, 0};
     uint32_t err = 0;
 
+    auto begin_scene = [&]() -> const SceneDev& {
+        if constexpr (NEAR) return sv[sc].scene;
+        else return tsc;
+    };
     auto add_sample = [&](float ci) {
         if (ci > 1.0f) acc = make_float4(acc.x + color.x, acc.y + color.y, acc.z + color.z, acc.w + 1.0f);
         else acc = make_float4(color.x, color.y, color.z, 1.0f);
@@ -97,7 +101,7 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
             color = mk(1.0f, 1.0f, 1.0f);
             bounce = 0;
             if (V.cp.depth > 0) {
-                walker_begin(w, tsc, ro, rd);
+                walker_begin(w, begin_scene(), ro, rd);
                 return B_TRAVERSE;
             }
             add_sample(V.cp.current_iteration + (float)k);
@@ -133,7 +137,6 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
                     sc = lo;
                     tsc.nodes = sv[sc].scene.nodes;
                     tsc.root_ref = sv[sc].scene.root_ref;
-                    tsc.nroot = sv[sc].scene.nroot;
                     tsc.watertight = sv[sc].scene.watertight;
                     gid = mine - sv[sc].pixel_begin;
                     rng.state = sv[sc].rng[gid];
@@ -196,7 +199,7 @@ batch_kernel(const BatchView* __restrict__ views, uint32_t nviews, uint32_t tota
                     cont = shade_hit<SEM, MATH_PORTABLE, false, !NEAR>(V.scene, V.cp, rng, h, &ro, &rd, &color, &scn);
                 }
                 if (cont && ++bounce < V.cp.depth) {
-                    walker_begin(w, tsc, ro, rd);
+                    walker_begin(w, begin_scene(), ro, rd);
                     mode = B_TRAVERSE;
                 } else {
                     add_sample(V.cp.current_iteration + (float)k);

@@ -27,15 +27,34 @@
 // accepted, and nothing replaces it.  A second candidate within T (a tie, or
 // two surfaces within a rounding step) sets `unsure`.
 //
-// What is pruned.  A box entered more than a margin behind the best t is
-// skipped.  For the reference to have accepted a primitive in there, the
-// primitive's computed t would have to lie that far in front of its own box:
-// a rounding error of more than kNearMargin of t plus 2^-10 of the
-// coordinates, against 2^-23 per operation.  Triangles whose shape alone can
-// magnify rounding that much (edges parallel to one part in 2^10) are given
-// their whole tree's box by the builder; for the others it takes a ray within
-// about 2^-13 of the triangle's plane whose garbage t also beats a surface of
-// the same place.
+// What is pruned.  A box entered beyond `lim` is skipped: T, plus what the
+// computed t of a primitive in there can lie in front of the computed entry of
+// its boxes.  That is, in units of t,
+//   * rounding of the slab test: 2^-23 of the origin's and the box's
+//     coordinates in the space of the test, times 1/d of the axis, for each of
+//     the two boxes compared.  A ray that runs along a box's face (|d| down to
+//     safe_invdir's 1e-5) and a mesh far from its own origin (survey data, that
+//     its transform brings back) make it large: the margin of a mesh is taken
+//     from the ray's origin in its space (near_move), the TLAS's from the ray's
+//     own (walker_begin, near_turn).
+//   * rounding of the shape's transform, which moves the hit against the box of
+//     the shape in the TLAS: near_turn and near_reach (tree_build.cu,
+//     shapes_kernel; also a box that is not quite around its shape).
+//   * rounding of the primitive's own test, across the ray (triangle_pad, in the
+//     place of a mesh leaf's type; near_reach) and along it (kNearSlide times
+//     that; kNearMargin of t).  Triangles whose shape alone can magnify rounding
+//     a thousandfold (edges parallel to one part in 2^10) are given their whole
+//     tree's box by the builder.
+// With a margin of 2^-10 of the world origin's coordinates alone, 215 of 1.6 M
+// rays at instances of a mesh modelled 10^6 from its origin missed what the
+// reference hits, and 41 of 0.7 M from the sphere field's surfaces with epsilon
+// zero; the margins cost 1 to 2 % of a frame (1080p scene 314 -> 320 ms).
+//
+// What is left: a ray in a triangle's plane, to within rounding, is given a t by
+// Möller and Trumbore's test that is rounding alone, anywhere along the ray, and
+// the reference's result is then a matter of whether it came to that triangle
+// before the true hit.  (0 of 10^8 rays in random directions and off surfaces; of
+// rays aimed along the planes of triangles in a random soup, 6 in 10^4.)
 #pragma once
 
 #include "pt_device.cuh"
@@ -54,7 +73,8 @@ struct NearWalker {
     int sp, floor;             // entries on the stack; those that are not of this space
     f3 o, d, inv, oxinv;       // (of the TLAS only while inner nodes of it are visited)
     float t, tie;              // best hit; T of the comment above
-    float lim, margin;         // boxes entered beyond `lim` are skipped; the origin's share of the margin
+    float lim;                 // boxes entered beyond are skipped
+    float margin, tlas_margin; // the share of it that does not grow with t: in this space, and in the TLAS
     uint32_t shape;            // current shape's node; kNearNone in the TLAS
     float entry;               // entry of its box
     uint32_t hit_shape, hit_tri;
@@ -96,21 +116,33 @@ __device__ __forceinline__ void near_space(NearWalker& w, f3 o, f3 d) {
     w.oxinv = mul(neg(o), w.inv);
 }
 
-__device__ __forceinline__ void walker_begin(NearWalker& w, const SceneDev& sc, f3 ro, f3 rd) {
-    w.node = sc.nroot;
+__device__ __forceinline__ float max_abs(f3 a) { return fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)); }
+
+__device__ __forceinline__ float min_abs(f3 a) { return fminf(fminf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)); }
+
+// The limit for the best hit of the moment.
+__device__ __forceinline__ float near_limit(const NearWalker& w) {
+    return w.tie + (w.tie * kNearMargin + w.margin);
+}
+
+__device__ __forceinline__ void near_start(NearWalker& w, uint32_t root, f3 ro, f3 rd) {
+    w.node = root;
     w.near = -INFINITY;
     w.sp = w.floor = 0;
     near_space(w, ro, rd);
     w.t = w.tie = (float)3.40282e+38;
     w.lim = INFINITY;
-    // 2^-10 of the origin's coordinates in units of t (over the direction's
-    // largest component); what t reaches from there is in kNearMargin's share
-    w.margin = fmaxf(fmaxf(fabsf(ro.x), fabsf(ro.y)), fabsf(ro.z)) * 0.0009765625f *
-               fminf(fminf(fabsf(w.inv.x), fabsf(w.inv.y)), fabsf(w.inv.z));
     w.shape = kNearNone;
     w.entry = -INFINITY;
     w.hit_shape = kNearNone;
     w.unsure = w.redo = w.away = false;
+}
+
+__device__ __forceinline__ void walker_begin(NearWalker& w, const SceneDev& sc, f3 ro, f3 rd) {
+    near_start(w, sc.nroot, ro, rd);
+    // (in units of t)
+    w.margin = w.tlas_margin = sc.near_slide * min_abs(w.inv) +
+                               (max_abs(ro) * (2.0f * sc.near_turn) + sc.near_reach) * max_abs(w.inv);
 }
 
 // aabb_hit_fast that also gives the entry.
@@ -138,7 +170,7 @@ __device__ __forceinline__ bool near_accept(NearWalker& w, float t, float near) 
     w.t = t;
     w.tie = tie;
     // (redo: the reference's own t_max)
-    w.lim = w.redo ? t : fmaxf(t + (fabsf(t) * kNearMargin + w.margin), tie);
+    w.lim = w.redo ? t : near_limit(w);
     return true;
 }
 
@@ -225,6 +257,8 @@ __device__ __forceinline__ bool near_move(NearWalker& w, const SceneDev& sc, f3 
             w.entry = -INFINITY;
             w.floor = 0;
             w.away = true;
+            w.margin = w.tlas_margin;
+            if (!w.redo) w.lim = near_limit(w);
             near_pop(w, stack);
         }
         if (w.node == kNearLeave) {
@@ -232,8 +266,7 @@ __device__ __forceinline__ bool near_move(NearWalker& w, const SceneDev& sc, f3 
             // few rays: ties and near-ties.  The same steps over the
             // reference's nodes, right child first, boxes tested against the
             // best t of the moment and never again
-            walker_begin(w, sc, ro, rd);
-            w.node = sc.root_ref;
+            near_start(w, sc.root_ref, ro, rd);
             w.redo = true;
             w.lim = w.t;
             return true;
@@ -241,6 +274,7 @@ __device__ __forceinline__ bool near_move(NearWalker& w, const SceneDev& sc, f3 
     }
     const uint32_t type = w.node >> 30;
     f3 o = ro, d = rd;
+    float across = 0.0f;
     if (type != ORN_NODE_INTERNAL) {
         Node nd;
         nd.load(sc.nodes + 4 * (size_t)(w.node & kRefIndexMask));
@@ -274,10 +308,15 @@ __device__ __forceinline__ bool near_move(NearWalker& w, const SceneDev& sc, f3 
             w.floor = w.sp;
             w.node = bits(nd.e.w);
             w.near = -INFINITY;
+            across = nd.c.w;
         }
     }
     w.away = false;
     near_space(w, o, d);
+    if (w.shape != kNearNone && !w.redo) {   // (a mesh was entered)
+        w.margin = max_abs(w.oxinv) * 0x1p-21f + across * (max_abs(w.inv) + kNearSlide * min_abs(w.inv));
+        w.lim = near_limit(w);
+    }
     return true;
 }
 

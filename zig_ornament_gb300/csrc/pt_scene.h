@@ -34,6 +34,9 @@ constexpr uint32_t kRefIndexMask = 0x3FFFFFFFu;
 // triangle id whose leaf box in its trees is not its own.
 constexpr int kNearStackSize = 64;
 constexpr uint32_t kNearOwnBox = 0x80000000u;
+// How much farther along a ray than across it the rounding of a triangle's test
+// is allowed to move the hit (rays at up to 2^-8 of a right angle from its plane).
+constexpr float kNearSlide = 256.0f;
 
 struct TexDesc {
     const unsigned char* data;
@@ -63,6 +66,10 @@ struct SceneDev {
     uint32_t near;
     uint32_t large;             // enough nodes that walking them outweighs shading
     uint32_t nroot;             // reference of the TLAS root
+    // What pruning in the TLAS allows for (tree_build.cu, shapes_kernel): 2^-20
+    // times the largest condition number of the shapes' transforms; how far from
+    // its shape's box a hit may be computed in any direction, and along the ray.
+    float near_turn, near_reach, near_slide;
 };
 
 }  // namespace orn

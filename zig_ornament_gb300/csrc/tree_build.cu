@@ -60,6 +60,9 @@ constexpr uint32_t kRoundsPerSync = 4;
 constexpr uint32_t kOwnBoxMark = 0x80000000u;   // a leaf's box is not its triangle's own
 constexpr uint32_t kMostSlivers = 64;
 constexpr float kSliver = 1024.0f;
+// What triangle_pad and shapes_kernel allow for.
+constexpr float kPadTriangle = 0x1p-20f, kPadMove = 0x1p-20f, kPadSphere = 0x1p-19f;
+constexpr double kMostMiss = 0x1p-12, kMostTurn = 0x1p12;
 constexpr uint32_t kNearDepthLimit = kNearStackSize;   // levels of TLAS and BLAS together (one entry each)
 
 // Counters and flags of one build (device; read back between phases).
@@ -68,6 +71,10 @@ struct State {
     uint32_t huge;
     uint32_t slivers;
     uint32_t prims;       // triangles that belong to a mesh, and reachable TLAS leaves
+    float turn;           // SceneDev::near_turn
+    float reach;          // of SceneDev::near_reach, the shapes' share
+    float slide;          // SceneDev::near_slide
+    float world;          // largest |coordinate| of the TLAS leaves' boxes
     uint32_t trees;       // meshes with triangles, and the TLAS
     uint32_t blas_depth, tlas_depth;
     uint32_t next_node;   // inner nodes made
@@ -216,12 +223,37 @@ __device__ __forceinline__ bool is_sliver(const orn_bvh_node& n) {
     return l1 * l2 > 0.0f && !(area * kSliver > l1 * l2);   // (a zero edge gives det = 0: never a hit)
 }
 
+// How far from the triangle, across the ray, the rounding of the reference's
+// test can put a hit: 2^-22 of the triangle's extent over the sine between its
+// edges, with a factor of 4 (what it is of the ray's length, the part of
+// kNearMargin covers).
+__device__ __forceinline__ float triangle_pad(const orn_bvh_node& n) {
+    float lo[3], hi[3];
+    triangle_box(n, lo, hi);
+    double e1[3], e2[3], l1 = 0.0, l2 = 0.0, cc = 0.0;
+    for (int k = 0; k < 3; ++k) {
+        e1[k] = (double)n.left_aabb_max_or_v1[k] - n.left_aabb_min_or_v0[k];
+        e2[k] = (double)n.right_aabb_min_or_v2[k] - n.left_aabb_min_or_v0[k];
+        l1 += e1[k] * e1[k];
+        l2 += e2[k] * e2[k];
+    }
+    for (int k = 0; k < 3; ++k) {
+        const int a = (k + 1) % 3, b = (k + 2) % 3;
+        const double c = e1[a] * e2[b] - e1[b] * e2[a];
+        cc += c * c;
+    }
+    if (!(cc > 0.0)) return 0.0f;   // (no area: never hit)
+    // (a sliver's box is its tree's, whatever its edges)
+    return fmaxf(fmaxf(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]) * kPadTriangle *
+           (float)fmin(sqrt(l1 * l2 / cc), (double)kSliver);
+}
+
 // Sort key and box of every primitive, by node index (BLAS, then TLAS).
 __global__ void prims_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t T, const orn_bvh_node* __restrict__ blas,
                              uint32_t B, const uint32_t* __restrict__ bparent, const uint32_t* __restrict__ tparent,
                              const uint8_t* __restrict__ is_root, unsigned long long* __restrict__ keys,
                              uint32_t* __restrict__ vals, float4* __restrict__ boxes, uint8_t* __restrict__ tree_used,
-                             State* st) {
+                             uint32_t* __restrict__ mesh_pad, State* st) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= B + T) return;
     keys[i] = 1ull << 60;   // after every tree: not a primitive of one
@@ -265,6 +297,7 @@ __global__ void prims_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t T, 
         float ext = 0.0f;
         for (int k = 0; k < 3; ++k) ext = fmaxf(ext, fmaxf(fabsf(lo[k]), fabsf(hi[k])));
         if (!(ext < 1e30f)) st->bad = 1u;
+        atomicMax((uint32_t*)&st->world, __float_as_uint(ext));
         const orn_bvh_node root = tlas[T - 1];
         if (T > 1) {
             float l2[3], h2[3];
@@ -311,11 +344,98 @@ __global__ void prims_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t T, 
             hi[k] = thi[k];
         }
     }
+    if (!top) {
+        const uint32_t pad = __float_as_uint(triangle_pad(nd));
+        if (pad > *(volatile uint32_t*)&mesh_pad[tree]) atomicMax(&mesh_pad[tree], pad);
+    }
     boxes[2 * (size_t)i] = make_float4(lo[0], lo[1], lo[2], 0.0f);
     boxes[2 * (size_t)i + 1] = make_float4(hi[0], hi[1], hi[2], own_box);
     atomicAdd(&st->prims, 1u);
     uint8_t* used = top ? tree_used + B : tree_used + tree;
     if (*used == 0) *used = 1;
+}
+
+// How far the hits that the reference's tests compute in a shape may lie outside
+// its box in the TLAS (the largest of all shapes, and of their axes, is
+// SceneDev::near_reach): by the padding of its triangles or its ball, by the
+// rounding of its inverse transform's translation, and because the box, a
+// caller's, is not quite around it.  The rounding that grows with the ray's
+// origin is near_turn's.  Boxes that miss their shapes altogether, and singular
+// transforms, keep the blob's walk.
+__global__ void shapes_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t T,
+                              const orn_bvh_node* __restrict__ blas, uint32_t B, const float4* __restrict__ xforms,
+                              const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ mesh_pad,
+                              const float4* __restrict__ boxes, State* st) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= T || keys[B + (size_t)i] >> 60 != 0ull) return;
+    const orn_bvh_node nd = tlas[i];
+    double a[3][3], t[3], inv[3][3];
+    for (int r = 0; r < 3; ++r) {
+        const float4 row = xforms[(size_t)nd.transform_id * 8 + r];
+        a[r][0] = row.x;
+        a[r][1] = row.y;
+        a[r][2] = row.z;
+        t[r] = row.w;
+    }
+    for (int r = 0; r < 3; ++r)
+        for (int c = 0; c < 3; ++c) {
+            const int a0 = (c + 1) % 3, a1 = (c + 2) % 3, b0 = (r + 1) % 3, b1 = (r + 2) % 3;
+            inv[r][c] = a[a0][b0] * a[a1][b1] - a[a0][b1] * a[a1][b0];
+        }
+    const double det = a[0][0] * inv[0][0] + a[0][1] * inv[1][0] + a[0][2] * inv[2][0];
+    const bool mesh = nd.node_type == ORN_NODE_MESH;
+    double centre[3] = {0.0, 0.0, 0.0}, half[3] = {1.0, 1.0, 1.0}, pad[3] = {kPadSphere, kPadSphere, kPadSphere};
+    if (mesh) {
+        const orn_bvh_node root = blas[nd.left_or_custom_id];
+        float lo[3], hi[3];
+        if (root.node_type == ORN_NODE_TRIANGLE) {
+            triangle_box(root, lo, hi);
+        } else {
+            float l2[3], h2[3];
+            stored_box(root, false, lo, hi);
+            stored_box(root, true, l2, h2);
+            for (int k = 0; k < 3; ++k) {
+                lo[k] = fminf(lo[k], l2[k]);
+                hi[k] = fmaxf(hi[k], h2[k]);
+            }
+        }
+        for (int k = 0; k < 3; ++k) {
+            centre[k] = 0.5 * ((double)lo[k] + hi[k]);
+            half[k] = 0.5 * ((double)hi[k] - lo[k]);
+            pad[k] = __uint_as_float(mesh_pad[nd.left_or_custom_id]);
+        }
+    }
+    const float4 blo = boxes[2 * ((size_t)B + i)], bhi = boxes[2 * ((size_t)B + i) + 1];
+    const double box_lo[3] = {blo.x, blo.y, blo.z}, box_hi[3] = {bhi.x, bhi.y, bhi.z};
+    double turn = 0.0, out = 0.0, slide = 0.0;
+    bool ok = true;
+    for (int r = 0; r < 3; ++r) {
+        double at = 0.0, reach = 0.0, square = 0.0, move = 0.0, wide = 0.0, cond = 0.0;
+        for (int c = 0; c < 3; ++c) {
+            const double v = inv[r][c] / det, m = fabs(v);
+            at += v * (centre[c] - t[c]);
+            reach += m * half[c];
+            square += m * m;
+            move += m * fabs(t[c]);
+            wide += m * pad[c];
+            cond += m * (fabs(a[c][0]) + fabs(a[c][1]) + fabs(a[c][2]));
+        }
+        if (!mesh) reach = sqrt(square);   // (the box of the ball's image)
+        if (mesh) slide = fmax(slide, wide * kNearSlide);
+        wide += (move + fabs(at) + reach) * kPadMove;
+        const double miss = fmax(at + reach - box_hi[r], box_lo[r] - (at - reach));
+        // (the only shape's box is not tested)
+        ok = ok && (T == 1 || miss <= kMostMiss * (fabs(box_lo[r]) + fabs(box_hi[r]) + move)) && cond < kMostTurn;
+        out = fmax(out, wide + fmax(miss, 0.0));
+        turn = fmax(turn, cond);
+    }
+    if (!ok) {   // (NaN among them)
+        st->bad = 1u;
+        return;
+    }
+    atomicMax((uint32_t*)&st->turn, __float_as_uint(__double2float_ru(turn * kPadMove)));
+    atomicMax((uint32_t*)&st->slide, __float_as_uint(__double2float_ru(slide)));
+    atomicMax((uint32_t*)&st->reach, __float_as_uint(__double2float_ru(T == 1 ? 0.0 : out)));
 }
 
 __global__ void count_trees_kernel(const uint8_t* __restrict__ used, uint32_t n, State* st) {
@@ -554,6 +674,7 @@ struct Emit {
     uint32_t first;            // index of the first new node
     uint32_t* root_of;         // by BLAS node index: the reference of a mesh's root
     uint32_t* mesh_place;      // places of the mesh leaves
+    const uint32_t* mesh_pad;  // by BLAS node index: triangle_pad of a mesh
     State* st;
 };
 
@@ -627,14 +748,18 @@ __global__ void write_kernel(Emit e, uint32_t total) {
     const uint32_t v = e.vals[c];
     const float4* src = e.nodes + 4 * (size_t)(v < e.B ? e.T + v : v - e.B);
     float4 a = src[0];
-    const float4 mid = src[2];
+    float4 mid = src[2];
     if (v < e.B && (__float_as_uint(e.node_box[2 * (size_t)c + 1].w) & kOwnBoxMark) != 0u)
         a.w = __uint_as_float(__float_as_uint(a.w) | kNearOwnBox);
+    if (v >= e.B && __float_as_uint(mid.w) == ORN_NODE_MESH) {
+        e.mesh_place[atomicAdd(&e.st->meshes, 1u)] = c;
+        // (in the place of the type, which references carry)
+        mid.w = __uint_as_float(e.mesh_pad[(__float_as_uint(src[3].w) & kRefIndexMask) - e.T]);
+    }
     o[0] = a;
     o[1] = src[1];
     o[2] = mid;
     o[3] = src[3];
-    if (v >= e.B && __float_as_uint(mid.w) == ORN_NODE_MESH) e.mesh_place[atomicAdd(&e.st->meshes, 1u)] = c;
 }
 
 // Points the mesh leaves of the written array at their new roots.
@@ -688,7 +813,9 @@ struct Build {
 };
 
 // Bytes of the first phase's arrays (all nodes), and of the second's (n primitives).
-size_t first_bytes(size_t T, size_t B) { return 64 * (T + B) + 4 * (T + B) + 2 * (B + 1) + 24 * (T + B) + 32 * (T + B) + 32 * 256; }
+size_t first_bytes(size_t T, size_t B) {
+    return 64 * (T + B) + 4 * (T + B) + 2 * (B + 1) + 24 * (T + B) + 32 * (T + B) + 4 * B + 32 * 256;
+}
 size_t second_bytes(size_t n, size_t T, size_t B, size_t temp) {
     return temp + 64 * n + 8 * n + 13 * n + 4 * (T + B) + 32 * 256;
 }
@@ -711,8 +838,11 @@ cudaError_t Build::near_trees(Arena& a) {
     uint32_t* vals = a.take<uint32_t>(N);
     uint32_t* vals2 = a.take<uint32_t>(N);
     float4* boxes = a.take<float4>(2 * (size_t)N);
+    uint32_t* mesh_pad = a.take<uint32_t>(B);   // by mesh: the largest of its triangles' (float bits)
+    WB(cudaMemsetAsync(mesh_pad, 0, 4 * (size_t)B, s));
     prims_kernel<<<blocks(N, 256), 256, 0, s>>>(tlas, T, blas, B, bparent, tparent, is_root, keys, vals, boxes, used,
-                                                d_state);
+                                                mesh_pad, d_state);
+    shapes_kernel<<<blocks(T, 128), 128, 0, s>>>(tlas, T, blas, B, xforms, keys, mesh_pad, boxes, d_state);
     count_trees_kernel<<<blocks((size_t)B + 1, 256), 256, 0, s>>>(used, B + 1, d_state);
     WB(cudaGetLastError());
     WB(read_state());
@@ -767,6 +897,7 @@ cudaError_t Build::near_trees(Arena& a) {
     e.nodes = nodes;
     e.root_of = a2.take<uint32_t>(B);
     e.mesh_place = a2.take<uint32_t>(T);
+    e.mesh_pad = mesh_pad;
     e.st = d_state;
     // a binary tree of k leaves has 2k - 1 nodes here as in the blob: the new
     // ones are no more than those (build_scene_trees makes room for them)
@@ -784,6 +915,9 @@ cudaError_t Build::near_trees(Arena& a) {
     WB(read_state());
     if (h.near_depth[0] + h.near_depth[1] > kNearDepthLimit) return cudaSuccess;
     scene->nroot = h.root;
+    scene->near_turn = h.turn;
+    scene->near_slide = h.slide;
+    scene->near_reach = h.reach + h.turn * h.world;
     scene->near = scene->large && h.area[0] < kGoodTrees * h.area[1] ? 1u : 2u;
     return cudaSuccess;
 }
