@@ -1,14 +1,14 @@
 // tree_build.cu — the device side of scene creation: the kernels' node array,
 // and the trees that pt_near.cuh traverses.
 //
-//   1. The blob's nodes go to the device as they are; one pass writes the
-//      kernels' node array (pt_scene.h), a second finds every node's parent
-//      and checks what the near-first traversal's proof of equal results
+//   1. The blob's nodes go to the device as they are.  A pass finds every node's
+//      parent and checks what the near-first traversal's proof of equal results
 //      needs: each stored box has its lower corner first and holds the boxes
-//      stored below it, a triangle's box is that of its vertices, no node has two parents, and no walk can
-//      need more than the reference's 64 stack entries.  A blob without one
-//      of these (other builders' padding, shared subtrees) keeps the
-//      reference's walk.
+//      stored below it, a triangle's box is that of its vertices, no node has
+//      two parents, and no walk can need more than the reference's 64 stack
+//      entries.  A blob without one of these (other builders' padding, shared
+//      subtrees) keeps the reference's walk, and so does one whose new trees do
+//      not fit in memory: nothing is allocated for good until they are decided.
 //   2. Every triangle finds the mesh it belongs to by its parents; triangles
 //      and TLAS leaves are sorted by (tree, Morton code of the box centre).
 //   3. Binary trees by parallel locally-ordered clustering (Meister and
@@ -18,8 +18,9 @@
 //      the same tree whose union box has the least area; pairs that pick each
 //      other merge.  The last kSmallClusters are merged by one block in
 //      shared memory.
-//   4. The nodes are written as they are numbered: leaves in Morton order,
-//      then inner nodes round by round.  (Treelets of eight stored together,
+//   4. The kernels' node array (pt_scene.h) is written: the blob's nodes, in
+//      place if they are all there is, and the new ones behind them as they are
+//      numbered: leaves in Morton order, then inner nodes round by round.  (Treelets of eight stored together,
 //      top-down: 77.2 against 77.0 ms for 16 passes of the 1080p scene, and
 //      creation 5.6 against 4.5 ms, of a small scene 1.3 against 0.6.)
 //
@@ -85,6 +86,8 @@ struct State {
     float area[2];        // of the inner nodes' children's boxes: the blob's BLASes, the new ones
 };
 
+static_assert(sizeof(State) <= 256, "the space before the types");
+
 // Adds a warp's half box areas (lanes without one: 0) to *sum.
 __device__ __forceinline__ void add_area(float* sum, float a) {
     for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
@@ -92,31 +95,33 @@ __device__ __forceinline__ void add_area(float* sum, float a) {
 }
 __device__ __forceinline__ float half_area(float x, float y, float z) { return x * y + y * z + z * x; }
 
-__device__ __forceinline__ uint32_t ref_of(const orn_bvh_node* nodes, uint32_t i, uint32_t offset) {
-    return (offset + i) | (nodes[i].node_type << 30);
+__global__ void types_kernel(const orn_bvh_node* __restrict__ nodes, uint32_t n, uint8_t* __restrict__ types) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) types[i] = (uint8_t)nodes[i].node_type;
 }
 
 // The kernels' node array.  A triangle keeps its vertices as given, so
 // triangles sharing an edge see the same floats (the watertight test relies
 // on it), and the two edges the reference's test subtracts on the fly
 // (bvh.hip.h:81-82) — the same single-precision subtractions.
-__global__ void relayout_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t T,
-                                const orn_bvh_node* __restrict__ blas, uint32_t B, const float4* __restrict__ xforms,
-                                float4* __restrict__ out, State* st) {
+// (`out` may be the blob's nodes themselves: a thread reads its own node, and of
+// others the types only.)
+__global__ void relayout_kernel(const orn_bvh_node* nodes, uint32_t T, uint32_t B, const uint8_t* __restrict__ types,
+                                const float4* __restrict__ xforms, float4* out, State* st) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= T + B) return;
     const bool top = i < T;
-    const orn_bvh_node n = top ? tlas[i] : blas[i - T];
+    const orn_bvh_node n = nodes[i];
+    auto ref = [&](uint32_t k) { return k | ((uint32_t)types[k] << 30); };
     const float* a = n.left_aabb_min_or_v0;
     const float* b = n.left_aabb_max_or_v1;
     const float* c = n.right_aabb_min_or_v2;
     const float* e = n.right_aabb_max_or_v3;
     float4* o = out + (size_t)i * 4;
     if (n.node_type == ORN_NODE_INTERNAL) {
-        const orn_bvh_node* src = top ? tlas : blas;
         const uint32_t off = top ? 0u : T;
-        o[0] = make_float4(a[0], a[1], a[2], __uint_as_float(ref_of(src, n.left_or_custom_id, off)));
-        o[1] = make_float4(b[0], b[1], b[2], __uint_as_float(ref_of(src, n.right_or_material_index, off)));
+        o[0] = make_float4(a[0], a[1], a[2], __uint_as_float(ref(off + n.left_or_custom_id)));
+        o[1] = make_float4(b[0], b[1], b[2], __uint_as_float(ref(off + n.right_or_material_index)));
         o[2] = make_float4(c[0], c[1], c[2], __uint_as_float(ORN_NODE_INTERNAL));
         o[3] = make_float4(e[0], e[1], e[2], 0.0f);
         bool ok = true;
@@ -131,7 +136,7 @@ __global__ void relayout_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t 
     } else {   // sphere / mesh leaf: inverse rows 0..2 inline
         const float4* m = xforms + (size_t)n.transform_id * 2 * 4;
         const float4 r0 = m[0], r1 = m[1], r2 = m[2];
-        const uint32_t root = n.node_type == ORN_NODE_MESH ? ref_of(blas, n.left_or_custom_id, T) : 0u;
+        const uint32_t root = n.node_type == ORN_NODE_MESH ? ref(T + n.left_or_custom_id) : 0u;
         o[0] = r0;
         o[1] = r1;
         o[2] = make_float4(r2.x, r2.y, r2.z, __uint_as_float(n.node_type));
@@ -170,7 +175,7 @@ __global__ void parents_kernel(const orn_bvh_node* __restrict__ nodes, uint32_t 
         stored_box(nd, side != 0, lo, hi);
         // (a sphere of negative radius has its box the wrong way round: the slab
         // test takes it as it is, but no box above it holds it)
-        for (int k = 0; k < 3; ++k) ok = ok && lo[k] <= hi[k];
+        for (int k = 0; k < 3; ++k) ok = ok && lo[k] <= hi[k] && lo[k] > -1e30f && hi[k] < 1e30f;
         const orn_bvh_node ch = nodes[c];
         if (ch.node_type == ORN_NODE_INTERNAL) {
             for (int s2 = 0; s2 < 2; ++s2) {
@@ -689,6 +694,14 @@ __device__ __forceinline__ uint32_t node_ref(const Emit& e, uint32_t c) {
 }
 
 // One cluster per tree is left: its root.
+__global__ void levels_kernel(const float4* __restrict__ node_box, const uint32_t* __restrict__ cluster, uint32_t trees,
+                              State* st) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= trees) return;
+    const uint32_t c = cluster[i];
+    const uint32_t levels = __float_as_uint(node_box[2 * (size_t)c + 1].w) & ~kOwnBoxMark;
+    atomicMax(&st->near_depth[__float_as_uint(node_box[2 * (size_t)c].w) == kTlasTree ? 1 : 0], levels);
+}
 __global__ void roots_kernel(Emit e, const uint32_t* __restrict__ cluster, uint32_t trees) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= trees) return;
@@ -696,8 +709,6 @@ __global__ void roots_kernel(Emit e, const uint32_t* __restrict__ cluster, uint3
     const uint32_t tree = __float_as_uint(e.node_box[2 * (size_t)c].w);
     if (tree == kTlasTree) e.st->root = node_ref(e, c);
     else e.root_of[tree] = node_ref(e, c);
-    const uint32_t levels = __float_as_uint(e.node_box[2 * (size_t)c + 1].w) & ~kOwnBoxMark;
-    atomicMax(&e.st->near_depth[tree == kTlasTree ? 1 : 0], levels);
 }
 
 // Half areas of the boxes that the blob's BLAS inner nodes hold.
@@ -797,31 +808,40 @@ struct Build {
     const orn_scene_blob* blob;
     const float4* xforms;
     SceneDev* scene;
-    std::vector<void*>* allocs;
     cudaStream_t s;
     State* d_state = nullptr;
     State h{};
     orn_bvh_node *tlas = nullptr, *blas = nullptr;
-    float4* nodes = nullptr;
-    void* second = nullptr;   // the second phase's arena
+    void *first = nullptr, *second = nullptr;   // arenas of near_trees
+    // the new trees as near_trees leaves them to write_trees; no nodes: none
+    Emit e{};
+    uint32_t* cluster = nullptr;
+    uint32_t trees = 0, total = 0;
 
     cudaError_t read_state() {
         WB(cudaMemcpyAsync(&h, d_state, sizeof(State), cudaMemcpyDeviceToHost, s));
         return cudaStreamSynchronize(s);
     }
-    cudaError_t near_trees(Arena& a);
+    cudaError_t near_trees();
+    cudaError_t write_trees(float4* nodes);
 };
 
 // Bytes of the first phase's arrays (all nodes), and of the second's (n primitives).
 size_t first_bytes(size_t T, size_t B) {
-    return 64 * (T + B) + 4 * (T + B) + 2 * (B + 1) + 24 * (T + B) + 32 * (T + B) + 4 * B + 32 * 256;
+    return 4 * (T + B) + 2 * (B + 1) + 24 * (T + B) + 32 * (T + B) + 4 * B + 32 * 256;
 }
 size_t second_bytes(size_t n, size_t T, size_t B, size_t temp) {
     return temp + 64 * n + 8 * n + 13 * n + 4 * (T + B) + 32 * 256;
 }
 
-cudaError_t Build::near_trees(Arena& a) {
+// Decides whether the scene has near-first trees, and builds them up to their
+// nodes.  Out of memory is an answer too: then it has none.
+cudaError_t Build::near_trees() {
     const uint32_t T = blob->tlas_nodes_len, B = blob->blas_nodes_len, N = T + B;
+    Arena a;
+    a.size = first_bytes(T, B);
+    WB(cudaMalloc((void**)&a.base, a.size));
+    first = a.base;
     uint32_t* bparent = a.take<uint32_t>(B);
     uint32_t* tparent = a.take<uint32_t>(T);
     uint8_t* is_root = a.take<uint8_t>((size_t)B + 1);
@@ -846,8 +866,9 @@ cudaError_t Build::near_trees(Arena& a) {
     count_trees_kernel<<<blocks((size_t)B + 1, 256), 256, 0, s>>>(used, B + 1, d_state);
     WB(cudaGetLastError());
     WB(read_state());
-    const uint32_t n = h.prims, trees = h.trees;
-    if (h.bad || h.huge || h.slivers > kMostSlivers || h.tlas_depth + h.blas_depth > kDepthLimit || n == 0 ||
+    const uint32_t n = h.prims;
+    trees = h.trees;
+    if (h.bad || h.slivers > kMostSlivers || h.tlas_depth + h.blas_depth > kDepthLimit || n == 0 ||
         2 * (uint64_t)N > kRefIndexMask)
         return cudaSuccess;
     size_t sort_bytes = 0, select_bytes = 0;
@@ -863,7 +884,7 @@ cudaError_t Build::near_trees(Arena& a) {
     WB(cub::DeviceRadixSort::SortPairs(temp, tb, keys, keys2, vals, vals2, (int)N, 0, 61, s));
     float4* node_box = a2.take<float4>(4 * (size_t)n);
     uint2* child = a2.take<uint2>(n);
-    uint32_t* cluster = a2.take<uint32_t>(n);
+    cluster = a2.take<uint32_t>(n);
     uint32_t* cluster2 = a2.take<uint32_t>(n);
     uint32_t* nn = a2.take<uint32_t>(n);
     uint8_t* keep_flag = a2.take<uint8_t>(n);
@@ -887,33 +908,38 @@ cudaError_t Build::near_trees(Arena& a) {
         WB(cudaFuncSetAttribute(small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallClusters)));
         small_kernel<<<1, kSmallBlock, sizeof(SmallClusters), s>>>(cluster, trees, n, node_box, child, d_state);
     }
-    Emit e;
     e.n = n;
     e.B = B;
     e.T = T;
     e.node_box = node_box;
     e.child = child;
     e.vals = vals2;
-    e.nodes = nodes;
     e.root_of = a2.take<uint32_t>(B);
     e.mesh_place = a2.take<uint32_t>(T);
     e.mesh_pad = mesh_pad;
     e.st = d_state;
-    // a binary tree of k leaves has 2k - 1 nodes here as in the blob: the new
-    // ones are no more than those (build_scene_trees makes room for them)
     e.first = N;
-    e.out = nodes + 4 * (size_t)N;
-    const uint32_t total = 2 * n - trees;
-    roots_kernel<<<blocks(trees, 128), 128, 0, s>>>(e, cluster, trees);
-    write_kernel<<<blocks(total, 256), 256, 0, s>>>(e, total);
-    meshes_kernel<<<blocks(T, 128), 128, 0, s>>>(e.out, T, e.root_of, e.mesh_place, d_state);
+    const uint32_t all = 2 * n - trees;   // (no more than N: a binary tree of k leaves has 2k - 1 nodes here as there)
+    levels_kernel<<<blocks(trees, 128), 128, 0, s>>>(node_box, cluster, trees, d_state);
     if (scene->large) {
         if (B) blob_area_kernel<<<blocks(B, 256), 256, 0, s>>>(blas, B, &d_state->area[0]);
-        if (total > n) near_area_kernel<<<blocks(total - n, 256), 256, 0, s>>>(e, total, &d_state->area[1]);
+        if (all > n) near_area_kernel<<<blocks(all - n, 256), 256, 0, s>>>(e, all, &d_state->area[1]);
     }
     WB(cudaGetLastError());
     WB(read_state());
-    if (h.near_depth[0] + h.near_depth[1] > kNearDepthLimit) return cudaSuccess;
+    if (h.near_depth[0] + h.near_depth[1] <= kNearDepthLimit) total = all;
+    return cudaSuccess;
+}
+
+// Writes the new trees behind the blob's nodes.
+cudaError_t Build::write_trees(float4* nodes) {
+    e.nodes = nodes;
+    e.out = nodes + 4 * (size_t)e.first;
+    roots_kernel<<<blocks(trees, 128), 128, 0, s>>>(e, cluster, trees);
+    write_kernel<<<blocks(total, 256), 256, 0, s>>>(e, total);
+    meshes_kernel<<<blocks(e.T, 128), 128, 0, s>>>(e.out, e.T, e.root_of, e.mesh_place, d_state);
+    WB(cudaGetLastError());
+    WB(read_state());
     scene->nroot = h.root;
     scene->near_turn = h.turn;
     scene->near_slide = h.slide;
@@ -927,41 +953,55 @@ cudaError_t Build::near_trees(Arena& a) {
 cudaError_t build_scene_trees(const orn_scene_blob* blob, const float4* d_xforms, SceneDev* scene, NodeFacts* facts,
                               std::vector<void*>* allocs, cudaStream_t s) {
     const uint32_t T = blob->tlas_nodes_len, B = blob->blas_nodes_len;
+    const size_t N = (size_t)T + B;
     Build b;
     b.blob = blob;
     b.xforms = d_xforms;
     b.scene = scene;
-    b.allocs = allocs;
     b.s = s;
-    void* nodes = nullptr;
-    WB(cudaMalloc(&nodes, 2 * ((size_t)T + B) * 64));
-    allocs->push_back(nodes);
-    b.nodes = (float4*)nodes;
-    scene->nodes = b.nodes;
     scene->near = 0u;
-    scene->large = (uint64_t)blob->tlas_nodes_len + blob->blas_nodes_len >= kLargeScene ? 1u : 0u;
-    Arena a;
-    a.size = first_bytes(T, B);
-    WB(cudaMalloc((void**)&a.base, a.size));
-    const cudaError_t e = [&]() -> cudaError_t {
+    scene->large = N >= kLargeScene ? 1u : 0u;
+    void *raw = nullptr, *own = nullptr, *both = nullptr;   // the blob's nodes; State and types; nodes with new trees
+    cudaError_t e = [&]() -> cudaError_t {
+        WB(cudaMalloc(&raw, N * 64));
+        WB(cudaMalloc(&own, 256 + N));
+        b.d_state = (State*)own;
+        uint8_t* types = (uint8_t*)own + 256;
+        b.tlas = (orn_bvh_node*)raw;
+        b.blas = b.tlas + T;
         // the transforms came through the default stream, which `s` does not wait for
         WB(cudaStreamSynchronize(nullptr));
-        b.d_state = a.take<State>(1);
-        b.tlas = a.take<orn_bvh_node>(T);
-        b.blas = a.take<orn_bvh_node>(B);
         WB(cudaMemsetAsync(b.d_state, 0, sizeof(State), s));
         WB(cudaMemcpyAsync(b.tlas, blob->tlas_nodes, (size_t)T * 64, cudaMemcpyHostToDevice, s));
         if (B) WB(cudaMemcpyAsync(b.blas, blob->blas_nodes, (size_t)B * 64, cudaMemcpyHostToDevice, s));
-        relayout_kernel<<<blocks((size_t)T + B, 256), 256, 0, s>>>(b.tlas, T, b.blas, B, d_xforms, b.nodes, b.d_state);
+        types_kernel<<<blocks(N, 256), 256, 0, s>>>(b.tlas, (uint32_t)N, types);
         WB(cudaGetLastError());
-        WB(b.near_trees(a));
-        WB(b.read_state());
+        cudaError_t grown = b.near_trees();
+        if (grown == cudaSuccess && b.total != 0u) grown = cudaMalloc(&both, (N + b.total) * 64);
+        if (grown == cudaErrorMemoryAllocation) {
+            (void)cudaGetLastError();
+            b.total = 0u;
+        } else if (grown != cudaSuccess) {
+            return grown;
+        }
+        float4* nodes = (float4*)(b.total != 0u ? both : raw);
+        relayout_kernel<<<blocks(N, 256), 256, 0, s>>>(b.tlas, T, B, types, d_xforms, nodes, b.d_state);
+        WB(cudaGetLastError());
+        if (b.total != 0u) WB(b.write_trees(nodes));
+        else WB(b.read_state());
         facts->huge = b.h.huge;
-        return cudaStreamSynchronize(s);
+        scene->nodes = nodes;
+        return cudaSuccess;
     }();
-    if (b.second) cudaFree(b.second);
-    const cudaError_t f = cudaFree(a.base);
-    return e != cudaSuccess ? e : f;
+    if (e != cudaSuccess) cudaStreamSynchronize(s);
+    void* kept = const_cast<float4*>(scene->nodes);
+    if (e == cudaSuccess) allocs->push_back(kept);
+    for (void* p : {raw, own, both, b.first, b.second}) {
+        if (!p || (e == cudaSuccess && p == kept)) continue;
+        const cudaError_t f = cudaFree(p);
+        if (e == cudaSuccess) e = f;
+    }
+    return e;
 }
 
 }  // namespace orn

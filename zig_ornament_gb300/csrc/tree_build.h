@@ -17,10 +17,9 @@ struct NodeFacts {
 };
 
 // Writes the kernels' node array (scene->nodes: TLAS, then BLAS, four
-// float4 each) from the blob's nodes and transforms on the device, and builds
-// the near-first trees beside it when the blob allows (scene->near).  Device arrays
-// that stay with the scene are appended to *allocs.  Everything runs on `s`,
-// finished on return.
+// float4 each) from the blob's nodes and transforms on the device, and behind
+// it the near-first trees when the blob allows and memory lasts (scene->near).
+// The array is appended to *allocs.  Everything runs on `s`, finished on return.
 cudaError_t build_scene_trees(const orn_scene_blob* blob, const float4* d_xforms, SceneDev* scene, NodeFacts* facts,
                               std::vector<void*>* allocs, cudaStream_t s);
 
