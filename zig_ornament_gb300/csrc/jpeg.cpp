@@ -263,16 +263,26 @@ struct Parser {
     uint32_t u8(size_t at) const { return data[at]; }
     uint32_t u16(size_t at) const { return ((uint32_t)data[at] << 8) | data[at + 1]; }
 
-    // Room for at least one more block's entries.  (Twice a coded byte's worth
-    // of entries to begin with; a start has to fit 32 bits, which 64 entries
-    // for each block of 2^28 pixels and several scans could exceed.)
+    // Room for at least one more block's entries.  To begin with, twice a coded
+    // byte's worth (a file may be mostly something else).  Entries that a second
+    // scan of a component has replaced are left behind, so that no number of
+    // scans needs more than twice what all blocks can have, which fits the 32
+    // bits of a start for 2^28 pixels.
     bool more_room() {
-        const size_t room = img->entry_room ? 2 * img->entry_room : std::max<size_t>(2 * len, 4096);
-        if (room > 0xFFFFFFFFull) return false;
+        size_t live = 0;
+        for (const Block& b : img->blocks) live += b.count;
+        const size_t most = 128 * img->blocks.size() + 64;
+        const size_t room = std::min(std::max<size_t>({img->entry_room, 2 * live, std::min(2 * len, most), 4096}), most);
         std::unique_ptr<uint32_t[]> p(new (std::nothrow) uint32_t[room]);
         if (!p) return false;
-        if (img->entry_count) std::memcpy(p.get(), img->entries.get(), img->entry_count * 4);
+        size_t at = 0;
+        for (Block& b : img->blocks) {
+            if (b.count) std::memcpy(p.get() + at, img->entries.get() + b.start, b.count * 4);
+            b.start = (uint32_t)at;
+            at += b.count;
+        }
         img->entries = std::move(p);
+        img->entry_count = at;
         img->entry_room = room;
         return true;
     }
