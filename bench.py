@@ -345,20 +345,19 @@ def roofline_block(bytes_per_launch, avg_launch_s, workload, clocks, profile_nam
     """The roofline object of a megakernel workload.
 
     L2-resident scenes (every workload but `large`): the kernel is bound by
-    the L1/TEX pipeline and issue slots (ncu: L1/TEX throughput and issue
-    activity near 60 %, DRAM below 1 %), so `achieved` (algorithmic bytes per
-    launch over the measured launch time) is set against the nominal L1 load
-    bandwidth, and the ncu figures of this build are quoted beside it.
-    The large scene (1.3 GB of nodes, L2 hit rate ~60 %) is bound by HBM
-    latency: `achieved` is the DRAM traffic of one launch over the launch
-    time, against the measured HBM copy bandwidth.  `traffic` = DRAM bytes
-    per node visit of the ncu capture of this build (a smaller launch of the
-    same scene) x this launch's node visits.
+    the L1/TEX pipeline and issue slots (ncu: both near 60 %, DRAM below
+    1 %), so `achieved` is the L1/TEX bytes of one launch over the launch
+    time, against the nominal L1 load bandwidth.  The large scene (1.3 GB of
+    nodes, L2 hit rate ~50 %) is bound by HBM latency: `achieved` is the DRAM
+    traffic of one launch over the launch time, against the measured HBM copy
+    bandwidth.  Bytes per launch = bytes per counted node visit of the ncu
+    capture of this build (a smaller launch of the same scene) x this launch's
+    counted visits; without a capture of this build there is none.
 
-    Visits and bytes are those of a counting render, which walks the
-    reference's trees.  The timed kernel's near-first trees need about half
-    the visits, so `achieved` is a rate of the reference's work, and DRAM
-    bytes per visit are per visit of the reference's walk."""
+    Visits are counted in a counting render, which walks the reference's
+    trees; the timed kernel's near-first trees need about half of them.  The
+    bytes that the reference's walk reads over the time are therefore
+    `reference_work`: a rate of that work, not of this kernel's traffic."""
     peak_hbm, kind = measured_peaks()
     algo = bytes_per_launch / avg_launch_s / 1e9
     fig, src = profile_figures(profile_name) if profile_name else (None, "no profile")
@@ -370,14 +369,17 @@ def roofline_block(bytes_per_launch, avg_launch_s, workload, clocks, profile_nam
     hbm["frac"] = hbm["achieved"] / peak_hbm if hbm["achieved"] else None
     if workload == "large":
         out = {"bound": "hbm", "achieved": hbm["achieved"], "peak": peak_hbm, "unit": "GB/s", "frac": hbm["frac"],
-               "traffic": traffic, "peak_kind": f"{kind} HBM copy",
-               "algorithmic": {"achieved": algo, "unit": "GB/s",
-                               "note": "node and shading bytes the algorithm reads, L1/L2-served ones included"}}
+               "traffic": traffic, "peak_kind": f"{kind} HBM copy"}
     else:
         l1 = l1_peak_gbs(clocks, device)
-        out = {"bound": "l1tex", "achieved": algo, "peak": l1, "unit": "GB/s", "frac": algo / l1,
-               "traffic": traffic, "peak_kind": "nominal L1 load bandwidth (128 B/clk/SM x SMs x max SM clock)",
-               "hbm": hbm}
+        per_visit = (fig or {}).get("l1tex_bytes_per_visit")
+        achieved = per_visit * visits_per_launch / avg_launch_s / 1e9 if per_visit and visits_per_launch else None
+        out = {"bound": "l1tex", "achieved": achieved, "peak": l1, "unit": "GB/s",
+               "frac": achieved / l1 if achieved else None, "traffic": traffic,
+               "peak_kind": "nominal L1 load bandwidth (128 B/clk/SM x SMs x max SM clock)", "hbm": hbm}
+    out["reference_work"] = {"achieved": algo, "unit": "GB/s",
+                             "note": "node and shading bytes of the reference's walk over the time; the near-first "
+                                     "trees need about half of its visits"}
     out["ncu"] = ({k: fig[k] for k in fig if k not in ("sources",)} if fig else None)
     out["ncu_source"] = src
     return out
