@@ -49,12 +49,20 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 }
 
 // Centroid bounds: keys of the minima in bounds[0..3), of the maxima in [3..6).
+// (A triangle whose first vertex is NaN stays out of them, as with std::min and
+// std::max: fminf and fmaxf, which drop a NaN, would let its other vertices
+// move every triangle's code.)
 __global__ void centroid_kernel(const float* __restrict__ tri, uint32_t n, uint32_t* __restrict__ bounds) {
     uint32_t lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0u, 0u, 0u};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float* v = tri + (size_t)i * 9;
         for (int k = 0; k < 3; ++k) {
-            const float c = 0.5f * (fminf(fminf(v[k], v[3 + k]), v[6 + k]) + fmaxf(fmaxf(v[k], v[3 + k]), v[6 + k]));
+            float mn = v[k], mx = v[k];
+            for (int j = 1; j < 3; ++j) {
+                mn = v[3 * j + k] < mn ? v[3 * j + k] : mn;
+                mx = v[3 * j + k] > mx ? v[3 * j + k] : mx;
+            }
+            const float c = 0.5f * (mn + mx);
             if (!(c == c)) continue;
             lo[k] = min(lo[k], float_key(c));
             hi[k] = max(hi[k], float_key(c));
