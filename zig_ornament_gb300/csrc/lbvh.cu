@@ -30,6 +30,7 @@ namespace orn {
 namespace {
 
 constexpr uint32_t kLeafBit = 0x80000000u;
+constexpr size_t kNodesAtOnce = 1u << 20;   // nodes of finished meshes that wait on the device (64 MB)
 
 __device__ __forceinline__ uint32_t expand_bits(uint32_t v) {
     v = (v * 0x00010001u) & 0xFF0000FFu;
@@ -259,13 +260,14 @@ __global__ void write_kernel(const float* __restrict__ tri, const unsigned long 
 
 int lbvh_build_all(const LbvhJob* jobs, size_t count) {
     int devices = 0;
-    size_t most = 0, nodes = 0;   // triangles of the largest mesh, nodes of all
+    size_t most = 0, nodes = 0;   // triangles of the largest mesh, nodes of all with more than one
     for (size_t j = 0; j < count; ++j) {
         if (jobs[j].n == 0) return ORN_ERR_EMPTY_SCENE;
         if (jobs[j].n >= (1u << 31)) return ORN_ERR_INVALID_ARGUMENT;   // node and sort indices are int
         most = std::max<size_t>(most, jobs[j].n);
-        nodes += 2 * (size_t)jobs[j].n - 1;
+        if (jobs[j].n > 1) nodes += 2 * (size_t)jobs[j].n - 1;
     }
+    const size_t room = std::min(nodes, std::max(kNodesAtOnce, 2 * most));   // nodes that the device holds
     if (count && (cudaGetDeviceCount(&devices) != cudaSuccess || devices == 0)) return ORN_ERR_NO_DEVICE;
     int st = ORN_OK;
     auto ok = [&](cudaError_t e) {
@@ -273,10 +275,10 @@ int lbvh_build_all(const LbvhJob* jobs, size_t count) {
         return st == ORN_OK;
     };
     // One allocation for all meshes: the working arrays for the largest, used
-    // by one mesh after another in stream order, and every mesh's nodes, which
-    // are copied back once all are queued (8 meshes of 35k triangles: an
-    // allocation per array and a wait per mesh took the builder 15.4 ms, this
-    // 11.1, with the host's share of both).
+    // by one mesh after another in stream order, and the nodes, which are copied
+    // back once as many meshes are queued as there is room for (8 meshes of 35k
+    // triangles: an allocation per array and a wait per mesh took the builder
+    // 15.4 ms, this 11.1, with the host's share of both).
     size_t temp_bytes = 0;
     if (most > 1 && !ok(cub::DeviceRadixSort::SortKeys(nullptr, temp_bytes, (const unsigned long long*)nullptr,
                                                        (unsigned long long*)nullptr, (int)most, 0, 64)))
@@ -292,7 +294,7 @@ int lbvh_build_all(const LbvhJob* jobs, size_t count) {
                  a_right = place(most * 4), a_lo = place(most * 4), a_hi = place(most * 4), a_arr = place(most * 4),
                  a_slot_int = place(most * 4), a_slot_leaf = place(most * 4), a_pint = place(most * 4),
                  a_pleaf = place(most * 4), a_boxes = place(most * 24), a_bounds = place(24), a_temp = place(temp_bytes),
-                 a_out = place(nodes * sizeof(orn_bvh_node));
+                 a_out = place(room * sizeof(orn_bvh_node));
     cudaStream_t s = nullptr;
     if (most > 1 && ok(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)) && ok(cudaMalloc((void**)&mem, used))) {
         float* d_tri = (float*)(mem + a_tri);
@@ -303,11 +305,24 @@ int lbvh_build_all(const LbvhJob* jobs, size_t count) {
                  *d_bounds = (uint32_t*)(mem + a_bounds);
         int *d_pint = (int*)(mem + a_pint), *d_pleaf = (int*)(mem + a_pleaf);
         float* d_boxes = (float*)(mem + a_boxes);
-        orn_bvh_node* d_out = (orn_bvh_node*)(mem + a_out);
+        orn_bvh_node* const d_first = (orn_bvh_node*)(mem + a_out);
+        orn_bvh_node* d_out = d_first;
+        size_t back = 0;   // meshes before this one are copied back
+        auto copy_back = [&](size_t end) {
+            d_out = d_first;
+            for (; back < end && st == ORN_OK; ++back) {
+                if (jobs[back].n == 1) continue;
+                const size_t k = 2 * (size_t)jobs[back].n - 1;
+                ok(cudaMemcpyAsync(jobs[back].out, d_out, k * sizeof(orn_bvh_node), cudaMemcpyDeviceToHost, s));
+                d_out += k;
+            }
+            d_out = d_first;
+        };
         for (size_t j = 0; j < count && st == ORN_OK; ++j) {
             const size_t nn = jobs[j].n, ni = nn - 1;
             const uint32_t n = jobs[j].n;
             if (n == 1) continue;
+            if ((size_t)(d_out - d_first) + 2 * nn - 1 > room) copy_back(j);
             const int B = 256;
             const unsigned gn = (unsigned)((nn + B - 1) / B), gall = (unsigned)((2 * nn - 1 + B - 1) / B);
             ok(cudaMemcpyAsync(d_tri, jobs[j].tri, nn * 36, cudaMemcpyHostToDevice, s));
@@ -332,13 +347,7 @@ int lbvh_build_all(const LbvhJob* jobs, size_t count) {
             ok(cudaGetLastError());
             d_out += 2 * nn - 1;
         }
-        d_out = (orn_bvh_node*)(mem + a_out);
-        for (size_t j = 0; j < count && st == ORN_OK; ++j) {
-            const size_t k = 2 * (size_t)jobs[j].n - 1;
-            if (jobs[j].n == 1) continue;
-            ok(cudaMemcpyAsync(jobs[j].out, d_out, k * sizeof(orn_bvh_node), cudaMemcpyDeviceToHost, s));
-            d_out += k;
-        }
+        copy_back(count);
         ok(cudaStreamSynchronize(s));
     }
     if (s) {
