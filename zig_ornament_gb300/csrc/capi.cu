@@ -1065,7 +1065,7 @@ int orn_trace_rays(orn_context* ctx, const orn_ray* rays, size_t count, orn_hit*
     // one allocation: rays, hits, then visits or (near-first trees) the list
     // of rays left to the reference's walk; kept with the context up to
     // kRayBytesKept, as a program that queries rays does so again
-    const bool near = ctx->scene.near && !ctx->scene.exact_slabs && !visits && count < 0xFFFFFFFFull;
+    const bool near = ctx->scene.near && !ctx->scene.exact_slabs && !visits && count <= orn::kTraceMostRays;
     const size_t ray_bytes = (count * sizeof(orn_ray) + 255) / 256 * 256, hit_bytes = count * sizeof(orn_hit);
     const size_t bytes = ray_bytes + hit_bytes + (count + 2) * sizeof(uint32_t);
     if (bytes > ctx->ray_bytes) {

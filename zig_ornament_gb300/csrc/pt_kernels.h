@@ -63,6 +63,9 @@ constexpr int kNearInner = ORN_NEAR_INNER;
 #define ORN_TRACE_STEPS 4
 #endif
 constexpr int kTraceFetch = ORN_TRACE_FETCH, kTraceSteps = ORN_TRACE_STEPS;
+// The longest list: the 32-bit count of rays handed out goes past the end by up
+// to 32 for each resident warp, and must not come round to the first ray again.
+constexpr uint32_t kTraceMostRays = 0xf0000000u;
 
 // Radiance-cache side of a cached megakernel launch.  Every pixel traces one
 // sample, with next-event estimation: at a lambertian vertex whose scattered
@@ -289,7 +292,7 @@ cudaError_t launch_wf_logic(const WaveLaunch& p, uint32_t iter, int semantics, i
 cudaError_t launch_wf_extend(const WaveLaunch& p, uint32_t iter, bool count, bool fast, cudaStream_t s);
 // Closest hits of a ray list: the reference's walk, with visits when asked
 // for; or, with `work` (count + 2 words of working memory, for scenes with
-// near-first trees and fewer than 2^32 - 1 rays), on those trees; `all_safe`:
+// near-first trees and at most kTraceMostRays rays), on those trees; `all_safe`:
 // every ray fits the FMNMX slab test.
 cudaError_t launch_trace_rays(const SceneDev& sc, float t_min, const float* rays, size_t count,
                               orn_hit* hits, uint32_t* visits, uint32_t* error, uint32_t* work, bool all_safe,
