@@ -337,7 +337,7 @@ void drop_graph(orn_batch* b) {
 // table (pinned) and the frame's pixel total.
 int prepare_frame(orn_batch* b, uint32_t* total_pixels, uint32_t* semantics, int* slabs) {
     uint64_t total = 0;
-    int all = orn::BATCH_NEAR;
+    orn::BatchWalk walk;
     uint32_t sem0 = 0;
     for (size_t i = 0; i < b->contexts.size(); ++i) {
         orn::BatchView v;
@@ -352,12 +352,12 @@ int prepare_frame(orn_batch* b, uint32_t* total_pixels, uint32_t* semantics, int
         v.pixel_begin = (uint32_t)total;
         total += (uint64_t)v.cp.width * v.cp.height;
         if (total >= 0xFFFFFFFFull) return bfail(b, ORN_ERR_INVALID_ARGUMENT, "batch frame too large");
-        all = std::min<int>(all, !f ? orn::BATCH_EXACT : (v.scene.near > 1u ? orn::BATCH_NEAR : orn::BATCH_FAST));
+        walk.add(v, f);
         b->h_views[i] = v;
     }
     *total_pixels = (uint32_t)total;
     *semantics = sem0;
-    *slabs = all;
+    *slabs = walk.slabs();
     return ORN_OK;
 }
 
@@ -548,7 +548,7 @@ int orn_batch_tune(orn_batch* b, const char* cache_path, orn_batch_config* chose
     // per context: the contexts' own images and progress are untouched.
     std::vector<orn::BatchView> saved(b->contexts.size());
     uint64_t total64 = 0, samples = 0;
-    int slabs = orn::BATCH_NEAR;
+    orn::BatchWalk walk;
     uint32_t sem = 0;
     for (size_t i = 0; i < b->contexts.size(); ++i) {
         bool f = false;
@@ -556,7 +556,7 @@ int orn_batch_tune(orn_batch* b, const char* cache_path, orn_batch_config* chose
         int dev = 0;
         int st = orn::batch_prepare(b->contexts[i], &saved[i], &f, &sm, &dev, b->stream, false);
         if (st) return bfail(b, st, orn_last_error(b->contexts[i]));
-        slabs = std::min<int>(slabs, !f ? orn::BATCH_EXACT : (saved[i].scene.near > 1u ? orn::BATCH_NEAR : orn::BATCH_FAST));
+        walk.add(saved[i], f);
         sem = sm;
         const uint32_t px = saved[i].cp.width * saved[i].cp.height;
         saved[i].pixel_begin = (uint32_t)total64;
@@ -564,6 +564,7 @@ int orn_batch_tune(orn_batch* b, const char* cache_path, orn_batch_config* chose
         samples += (uint64_t)px * saved[i].spp;
     }
     if (total64 >= 0xFFFFFFFFull) return bfail(b, ORN_ERR_INVALID_ARGUMENT, "batch frame too large");
+    const int slabs = walk.slabs();
     const uint32_t total = (uint32_t)total64;
     char dev_name[256] = {0};
     cudaDeviceProp prop;

@@ -44,6 +44,25 @@ struct BatchConfig {
 // form, or the near-first trees (which imply that form).
 enum { BATCH_EXACT = 0, BATCH_FAST = 1, BATCH_NEAR = 2 };
 
+// What a batch walks: the near-first trees where all contexts have them and
+// those that gain by it have more samples to take than the others.  (A
+// context that does not gain loses up to 15 %, one that does gains 5 to 50; taken
+// only when all gain, one SAH tree kept a batch of any others from it.)
+struct BatchWalk {
+    bool fast = true, near = true;
+    double gain = 0.0, lose = 0.0;
+    void add(const BatchView& v, bool fast_slabs) {
+        fast = fast && fast_slabs;
+        near = near && v.scene.near != 0u;
+        const double work = (double)v.cp.width * v.cp.height * v.spp;
+        (v.scene.near > 1u ? gain : lose) += work;
+    }
+    int slabs() const {
+        if (!fast) return BATCH_EXACT;
+        return near && gain > lose ? BATCH_NEAR : BATCH_FAST;
+    }
+};
+
 // Launches one batched frame (views already in device memory).
 cudaError_t launch_batch(const BatchView* views, uint32_t nviews, uint32_t total_pixels, uint32_t* work_counter,
                          uint32_t* error, int semantics, int slabs, const BatchConfig& cfg, cudaStream_t s);
