@@ -248,11 +248,11 @@ typedef struct orn_context orn_context;
  * of the blob.  Validates every index in the blob.  Where the blob's boxes
  * contain what is below them and the trees have at most 64 levels, a second
  * set of trees over the same primitives is built beside the blob's (as much
- * memory again as its nodes), which plain renders and ray queries walk nearest
- * box first (orn_near_trees).  The hits are those of the blob's trees, but
- * where a ray runs in a triangle's plane, to within rounding: the reference's
- * test then gives a t that is rounding alone, and which surface such a ray hits
- * depends on the order of its visits. */
+ * memory again as its nodes), which ray queries and, where it is faster, plain
+ * renders walk nearest box first (orn_near_trees).  The hits are those of the
+ * blob's trees, but where a ray runs in a triangle's plane, to within rounding:
+ * the reference's test then gives a t that is rounding alone, and which surface
+ * such a ray hits depends on the order of its visits. */
 int orn_create(const orn_scene_blob* blob, int device, orn_context** out);
 
 /* PathTracer.deinit — src/hip_backend/path_tracer.zig:88-101. */
@@ -338,9 +338,11 @@ int orn_peek_constant_params(const orn_context* ctx, orn_constant_params* out);
 int orn_trace_rays(orn_context* ctx, const orn_ray* rays, size_t count,
                    orn_hit* hits, uint32_t* visits);
 
-/* Which trees this context's plain renders and ray queries walk (with the
- * present state; see orn_create): 0 the blob's; 1 renders the blob's, ray
- * queries without visits the second set; 2 both the second set. */
+/* Who walks the second set of trees (with the present state; see orn_create):
+ * 0 nobody; 1 ray queries without visits; 2 also orn_render_f64, and batches
+ * (orn_batch_render) where such contexts have the most to walk; 3 also
+ * orn_render with the megakernel; 4 also with the persistent wavefront.  Where
+ * the blob's trees are good, or little is to be walked, walking them is faster. */
 int orn_near_trees(const orn_context* ctx, uint32_t* out);
 
 /* Work counters of the last orn_render (zeros unless enabled with

@@ -21,13 +21,13 @@ def _rays(extent, n=200_000, seed=11):
     return np.concatenate([o, d], 1).astype(F32)
 
 
-def _assert_same_hits(scene, extent, epsilon=0.001, trees=2, middle=0.0):
+def _assert_same_hits(scene, extent, epsilon=0.001, trees=True, middle=0.0):
     """Rays in a cube about `middle`, and a bounce from what they hit."""
     r = ornament.Renderer(ornament.Bvh(scene), device=0)
     state = ornament.State()
     state.setRayCastEpsilon(epsilon)
     r.set_state(state.to_struct())
-    assert r.near_trees() == trees
+    assert (r.near_trees() > 0) == trees
     rays = _rays(extent)
     rays[:, :3] += F32(middle)
     hit = 0
@@ -51,10 +51,10 @@ def test_negative_radii():
     for i in range(30):
         r = rs.uniform(0.3, 1.2)
         s.createSphere((*rs.uniform(-4, 4, 3), 1), -r if i % 3 == 0 else r, grey)
-    _assert_same_hits(s, 5.0, trees=0)
+    _assert_same_hits(s, 5.0, trees=False)
 
 
-@pytest.mark.parametrize("epsilon,trees", [(1.0, 2), (-0.001, 0), (-5.0, 0), (float("nan"), 0)])
+@pytest.mark.parametrize("epsilon,trees", [(1.0, True), (-0.001, False), (-5.0, False), (float("nan"), False)])
 def test_ray_cast_epsilon(epsilon, trees):
     """The near-first trees are walked for hits from the origin on, not for hits behind it."""
     _assert_same_hits(scenes.spheres_scene(), 12.0, epsilon, trees)
@@ -115,7 +115,7 @@ def test_instances_of_many_sizes():
     _assert_same_hits(_terrains(300.0, 0.25, 6.0, scales=(0.01, 0.1, 1.0, 10.0)), 6.0)
 
 
-@pytest.mark.parametrize("change,trees", [("shrunk", 0), ("moved", 0), ("grown", 2)])
+@pytest.mark.parametrize("change,trees", [("shrunk", False), ("moved", False), ("grown", True)])
 def test_boxes_of_shapes_as_a_caller_gives_them(change, trees):
     """The boxes of shapes come from the caller, who can give any: with one that does
     not hold its shape, what a ray hits depends on the order of its visits."""

@@ -45,7 +45,7 @@ struct BatchConfig {
 enum { BATCH_EXACT = 0, BATCH_FAST = 1, BATCH_NEAR = 2 };
 
 // What a batch walks: the near-first trees where all contexts have them and
-// those that gain by it have more samples to take than the others.  (A
+// those that gain by it (NEAR_BATCH) have more to walk than the others.  (A
 // context that does not gain loses up to 15 %, one that does gains 5 to 50; taken
 // only when all gain, one SAH tree kept a batch of any others from it.)
 struct BatchWalk {
@@ -53,9 +53,9 @@ struct BatchWalk {
     double gain = 0.0, lose = 0.0;
     void add(const BatchView& v, bool fast_slabs) {
         fast = fast && fast_slabs;
-        near = near && v.scene.near != 0u;
-        const double work = (double)v.cp.width * v.cp.height * v.spp;
-        (v.scene.near > 1u ? gain : lose) += work;
+        near = near && v.scene.near != NEAR_NONE;
+        const double work = (double)v.cp.width * v.cp.height * v.spp * (1.0 + v.scene.visits);
+        (v.scene.near >= NEAR_BATCH ? gain : lose) += work;
     }
     int slabs() const {
         if (!fast) return BATCH_EXACT;

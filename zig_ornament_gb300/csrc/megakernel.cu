@@ -802,7 +802,7 @@ cudaError_t launch_mega_cached(const RenderLaunch& p, int semantics, bool fast, 
 
 template <int SEM>
 static cudaError_t launch_mega_t(const RenderLaunch& p, bool count, bool fast, cudaStream_t s) {
-    if (fast && !count && p.scene.near > 1u)
+    if (fast && !count && p.scene.near >= NEAR_MEGA)
         return launch_mega_tt<SEM, MATH_PORTABLE, false, true, false, false, false, true>(p, s);
     if (fast) return count ? launch_mega_tt<SEM, MATH_PORTABLE, true, true>(p, s)
                            : launch_mega_tt<SEM, MATH_PORTABLE, false, true>(p, s);
@@ -811,7 +811,7 @@ static cudaError_t launch_mega_t(const RenderLaunch& p, bool count, bool fast, c
 }
 
 cudaError_t launch_mega_f64(const RenderLaunch& p, int semantics, bool fast, cudaStream_t s) {
-    if (fast && p.scene.near > 1u)
+    if (fast && p.scene.near >= NEAR_BATCH)
         return semantics == SEM_WGSL ? launch_mega_tt<SEM_WGSL, MATH_PORTABLE, false, true, true, false, false, true>(p, s)
                                      : launch_mega_tt<SEM_HIP, MATH_PORTABLE, false, true, true, false, false, true>(p, s);
     if (semantics == SEM_WGSL)

@@ -38,6 +38,11 @@ constexpr uint32_t kNearOwnBox = 0x80000000u;
 // is allowed to move the hit (rays at up to 2^-8 of a right angle from its plane).
 constexpr float kNearSlide = 256.0f;
 
+// Who walks a scene's near-first trees (tree_build.cu, near_level): nobody; ray
+// lists; batches and the FP64 renderer too; the megakernel too; the persistent
+// wavefront too.
+enum { NEAR_NONE = 0, NEAR_RAYS = 1, NEAR_BATCH = 2, NEAR_MEGA = 3, NEAR_WAVE = 4 };
+
 struct TexDesc {
     const unsigned char* data;
     uint32_t width, height, pitch, format;
@@ -59,17 +64,17 @@ struct SceneDev {
     uint32_t textures_len;
     uint32_t watertight;        // 1: watertight triangle test (orn_state.triangle_test), 0: the reference's
     // Other trees over the same primitives (tree_build.cu), for the traversal
-    // of pt_near.cuh: behind the nodes above in the same array and format.
-    // `near` is 0 when the scene's arrays do not have what its proof of equal
-    // results needs, and the nodes above are then walked everywhere; 1 when the
-    // nodes above are good trees themselves, which renders walk faster; else 2.
-    uint32_t near;
+    // of pt_near.cuh: behind the nodes above in the same array and format, or
+    // NEAR_NONE when the scene's arrays do not have what its proof of equal
+    // results needs.
+    uint32_t near;              // which kernels walk them: NEAR_*
     uint32_t large;             // enough nodes that walking them outweighs shading
     uint32_t nroot;             // reference of the TLAS root
     // What pruning in the TLAS allows for (tree_build.cu, shapes_kernel): 2^-20
     // times the largest condition number of the shapes' transforms; how far from
     // its shape's box a hit may be computed in any direction, and along the ray.
     float near_turn, near_reach, near_slide;
+    float visits;               // that a ray is expected to make in the blob's trees (where the others were built)
 };
 
 }  // namespace orn

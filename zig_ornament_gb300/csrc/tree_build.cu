@@ -20,11 +20,13 @@
 //      shared memory.
 //   4. The kernels' node array (pt_scene.h) is written: the blob's nodes, in
 //      place if they are all there is, and the new ones behind them as they are
-//      numbered: leaves in Morton order, then inner nodes round by round.  (Treelets of eight stored together,
-//      top-down: 77.2 against 77.0 ms for 16 passes of the 1080p scene, and
-//      creation 5.6 against 4.5 ms, of a small scene 1.3 against 0.6.)
+//      numbered: leaves in Morton order, then inner nodes round by round.
+//      (Treelets of eight stored together, top-down: 77.2 against 77.0 ms for 16
+//      passes of the 1080p scene, and creation 5.6 against 4.5 ms, of a small
+//      scene 1.3 against 0.6.)
 //
-// Results do not depend on these trees, only speed does.
+// Results do not depend on these trees (pt_near.cuh has the exception), only
+// speed does; near_level has who walks them.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_select.cuh>
 
@@ -39,18 +41,11 @@ namespace {
 
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr uint32_t kTlasTree = 0x3fffffffu;   // tree id of the TLAS (meshes: their root's BLAS index)
-// Scenes of this many nodes (1 MB, more than an L1) are taken to spend more on
-// walking than on shading: the sphere field (975) and rooms (40) do not, the
-// mesh scenes (563 k and 2 M) do.
+// Cached frames of scenes of this many nodes (1 MB, more than an L1) are taken to
+// spend more on walking than on shading, and keep the shading code of their own
+// (SplitGeom).  Measured from 40 to 563 k nodes; on either side of the line what
+// is taken there is the faster one or within 1 %.
 constexpr uint32_t kLargeScene = 16384;
-// A large scene's renders stay on the blob's trees when the boxes of their
-// BLASes have less than this many times the near-first trees' area.  Binned-SAH
-// trees have 0.92, GPU-built linear ones 1.08 to 1.10, the reference's median
-// splits 1.77 to 1.84.  The first two are as good, and the reference's walk
-// costs less per visit (1080p scene of 16 passes, blob's trees against
-// near-first: SAH 65.7 and 76.8 ms, linear 70.1 and 76.9, reference 91.3 and
-// 77.0).  Ray lists, where latency counts, always take the near-first trees.
-constexpr float kGoodTrees = 1.35f;
 constexpr uint32_t kDepthLimit = 64;          // the reference's stack entries
 constexpr int kRadius = 16;
 constexpr int kNnBlock = 256;
@@ -83,7 +78,9 @@ struct State {
     uint32_t clusters;    // left to merge
     uint32_t near_depth[2];   // levels of the deepest BLAS, and of the TLAS
     uint32_t root;        // reference of the TLAS root
-    float area[2];        // of the inner nodes' children's boxes: the blob's BLASes, the new ones
+    uint32_t shapes_box[6];   // keys of the corners of the ordinary shapes' box (ordinary_kernel)
+    uint32_t large_shapes;   // left out of it
+    float visits[4];      // expected of a ray: the blob's TLAS and BLASes, the new ones
 };
 
 static_assert(sizeof(State) <= 256, "the space before the types");
@@ -711,31 +708,105 @@ __global__ void roots_kernel(Emit e, const uint32_t* __restrict__ cluster, uint3
     else e.root_of[tree] = node_ref(e, c);
 }
 
-// Half areas of the boxes that the blob's BLAS inner nodes hold.
-__global__ void blob_area_kernel(const orn_bvh_node* __restrict__ blas, uint32_t n, float* sum) {
+// ---- how much there is to walk -----------------------------------------------------------------
+// Visits that a ray is expected to make: a box is visited with the chance of its
+// area over that of the box of all shapes, a node in a mesh with that of its
+// mesh's instances times its area over the mesh's own.  Shapes that take up more
+// than a quarter of the scene (the ground, the walls of a room) would make all
+// others look out of the way, where rays hardly are: they are left out of the box
+// of all shapes, and no chance is more than one.
+__device__ __forceinline__ float inner_area(const orn_bvh_node& nd) {   // of the box around both children's
+    float lo[3], hi[3], l2[3], h2[3];
+    stored_box(nd, false, lo, hi);
+    stored_box(nd, true, l2, h2);
+    return half_area(fmaxf(hi[0], h2[0]) - fminf(lo[0], l2[0]), fmaxf(hi[1], h2[1]) - fminf(lo[1], l2[1]),
+                     fmaxf(hi[2], h2[2]) - fminf(lo[2], l2[2]));
+}
+__device__ __forceinline__ uint32_t order_key(float f) {   // order-preserving, for atomic maxima
+    const uint32_t u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float key_float(uint32_t k) {
+    return __uint_as_float((k & 0x80000000u) ? k & 0x7fffffffu : ~k);
+}
+__global__ void ordinary_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t T, uint32_t B,
+                                const unsigned long long* __restrict__ keys, const float4* __restrict__ boxes, State* st) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= T || keys[B + (size_t)i] >> 60 != 0ull) return;
+    const float4 lo = boxes[2 * ((size_t)B + i)], hi = boxes[2 * ((size_t)B + i) + 1];
+    if (T > 1 && half_area(lo, hi) > 0.25f * inner_area(tlas[T - 1])) {
+        atomicAdd(&st->large_shapes, 1u);
+        return;
+    }
+    const float v[6] = {-lo.x, -lo.y, -lo.z, hi.x, hi.y, hi.z};
+    for (int k = 0; k < 6; ++k) atomicMax(&st->shapes_box[k], order_key(v[k]));
+}
+__device__ __forceinline__ float shapes_area(const State* st, const orn_bvh_node& root) {
+    float v[6];
+    for (int k = 0; k < 6; ++k) {
+        const uint32_t key = st->shapes_box[k];
+        if (key == 0u) return inner_area(root);   // none
+        v[k] = key_float(key);
+    }
+    return half_area(v[3] + v[0], v[4] + v[1], v[5] + v[2]);
+}
+__device__ __forceinline__ float chance_of(float area, float all) { return all > 0.0f ? fminf(area / all, 1.0f) : 1.0f; }
+// Of each mesh (by its root): the sum over its instances.
+__global__ void chances_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t T, uint32_t B,
+                               const unsigned long long* __restrict__ keys, const float4* __restrict__ boxes,
+                               float* __restrict__ chance, const State* st) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= T || tlas[i].node_type != ORN_NODE_MESH || keys[B + (size_t)i] >> 60 != 0ull) return;
+    const float all = T > 1 ? shapes_area(st, tlas[T - 1]) : 0.0f;
+    atomicAdd(&chance[tlas[i].left_or_custom_id],
+              chance_of(half_area(boxes[2 * ((size_t)B + i)], boxes[2 * ((size_t)B + i) + 1]), all));
+}
+__global__ void blob_visits_kernel(const orn_bvh_node* __restrict__ tlas, uint32_t T,
+                                   const orn_bvh_node* __restrict__ blas, uint32_t B,
+                                   const uint32_t* __restrict__ bparent, const uint8_t* __restrict__ is_root,
+                                   const float* __restrict__ chance, State* st) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool top = i < T;
     float a = 0.0f;
-    if (i < n && blas[i].node_type == ORN_NODE_INTERNAL)
+    if (i < T + B && (top ? tlas[i] : blas[i - T]).node_type == ORN_NODE_INTERNAL) {
+        const orn_bvh_node nd = top ? tlas[i] : blas[i - T];
+        float all, times = 1.0f;
+        if (top) {
+            all = shapes_area(st, tlas[T - 1]);
+        } else {
+            uint32_t root = i - T;
+            for (uint32_t level = 0; !is_root[root] && bparent[root] != kNone && level < kDepthLimit; ++level)
+                root = bparent[root] & 0x7fffffffu;
+            all = inner_area(blas[root]);
+            times = is_root[root] ? chance[root] : 0.0f;
+        }
         for (int side = 0; side < 2; ++side) {
             float lo[3], hi[3];
-            stored_box(blas[i], side != 0, lo, hi);
-            a += half_area(hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2]);
-        }
-    add_area(sum, a);
-}
-// The same of the new BLAS nodes: those that are not the TLAS's.
-__global__ void near_area_kernel(Emit e, uint32_t total, float* sum) {
-    const uint32_t c = e.n + blockIdx.x * blockDim.x + threadIdx.x;
-    float a = 0.0f;
-    if (c < total) {
-        const uint2 ch = e.child[c - e.n];
-        for (int side = 0; side < 2; ++side) {
-            const uint32_t k = side ? ch.y : ch.x;
-            const float4 lo = e.node_box[2 * (size_t)k], hi = e.node_box[2 * (size_t)k + 1];
-            if (__float_as_uint(lo.w) != kTlasTree) a += half_area(hi.x - lo.x, hi.y - lo.y, hi.z - lo.z);
+            stored_box(nd, side != 0, lo, hi);
+            a += times * chance_of(half_area(hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2]), all);
         }
     }
-    add_area(sum, a);
+    add_area(&st->visits[0], top ? a : 0.0f);
+    add_area(&st->visits[1], top ? 0.0f : a);
+}
+__global__ void near_visits_kernel(Emit e, uint32_t total, const orn_bvh_node* __restrict__ tlas,
+                                   const orn_bvh_node* __restrict__ blas, const float* __restrict__ chance) {
+    const uint32_t c = e.n + blockIdx.x * blockDim.x + threadIdx.x;
+    float a = 0.0f;
+    bool top = false;
+    if (c < total) {
+        const uint2 ch = e.child[c - e.n];
+        const uint32_t tree = __float_as_uint(e.node_box[2 * (size_t)c].w);
+        top = tree == kTlasTree;
+        const float all = top ? shapes_area(e.st, tlas[e.T - 1]) : inner_area(blas[tree]);
+        for (int side = 0; side < 2; ++side) {
+            const uint32_t k = side ? ch.y : ch.x;
+            a += chance_of(half_area(e.node_box[2 * (size_t)k], e.node_box[2 * (size_t)k + 1]), all);
+        }
+        if (!top) a *= chance[tree];
+    }
+    add_area(&e.st->visits[2], top ? a : 0.0f);
+    add_area(&e.st->visits[3], top ? 0.0f : a);
 }
 
 __global__ void write_kernel(Emit e, uint32_t total) {
@@ -828,10 +899,39 @@ struct Build {
 
 // Bytes of the first phase's arrays (all nodes), and of the second's (n primitives).
 size_t first_bytes(size_t T, size_t B) {
-    return 4 * (T + B) + 2 * (B + 1) + 24 * (T + B) + 32 * (T + B) + 4 * B + 32 * 256;
+    return 4 * (T + B) + 2 * (B + 1) + 24 * (T + B) + 32 * (T + B) + 8 * B + 32 * 256;
 }
 size_t second_bytes(size_t n, size_t T, size_t B, size_t temp) {
     return temp + 64 * n + 8 * n + 13 * n + 4 * (T + B) + 32 * 256;
+}
+
+// Who walks the near-first trees.  They take fewer visits, but a visit costs
+// more: some 1.2 times as much in batches and the FP64 renderer, 1.5 times in the
+// megakernel and the persistent wavefront.  So the lines lie at `blob`, the visits
+// expected in the blob's trees, and at how many `times` those in the new ones that
+// is.  Measured with 960 x 540 pixels, 16 passes, 58 scenes of 9 to 2 M nodes on
+// the reference's median splits (1.0 to 2.0 times the visits), binned SAH (0.91 to
+// 1.1) and linear trees (0.93 to 1.2); time on the blob's trees over time on the new:
+//   * Ray lists, 1 to 1 M rays: 0.97 to 2.6, all scenes.
+//   * Spheres and walls of two triangles, where little of the walk is in meshes,
+//     and small meshes on a ground: shading counts for more, and the kernels on the
+//     new trees have it in one sequence (shade_geom).  Megakernel 0.98 to 1.61
+//     whatever the trees, batches 0.96 to 1.53; the wavefront, whose shading is the
+//     same on either, 0.78 to 1.05.  With fewer than four visits there is nothing
+//     to gain (five spheres: 1.0 to 1.09, batches 0.86 to 0.91).
+//   * Others, megakernel: from 1.5 times and 50 visits on 1.01 to 1.21 (a closed
+//     room of 64 instances 0.93); below that 0.64 to 1.25.
+//   * Wavefront: from 1.5 times and 200 visits on 1.03 to 1.24, below 0.66 to 1.21.
+//   * Batches: from 1.15 times on 1.0 to 1.6, below 0.88 to 1.25; FP64 likewise.
+// (One line for all, and none below 16,384 nodes, had frames of SAH and linear
+// trees there up to 1.35 times as long as on the blob's.)
+uint32_t near_level(const State& h) {
+    const float blob = h.visits[0] + h.visits[1], times = blob / (h.visits[2] + h.visits[3]);
+    const float in_meshes = h.visits[1] / blob;
+    if (!(blob >= 4.0f)) return NEAR_RAYS;
+    if (in_meshes <= 0.45f || (in_meshes <= 0.7f && blob <= 30.0f && h.large_shapes == 1u)) return NEAR_MEGA;
+    if (times >= 1.5f && blob >= 50.0f) return blob >= 200.0f ? NEAR_WAVE : NEAR_MEGA;
+    return times >= 1.15f ? NEAR_BATCH : NEAR_RAYS;
 }
 
 // Decides whether the scene has near-first trees, and builds them up to their
@@ -859,7 +959,9 @@ cudaError_t Build::near_trees() {
     uint32_t* vals2 = a.take<uint32_t>(N);
     float4* boxes = a.take<float4>(2 * (size_t)N);
     uint32_t* mesh_pad = a.take<uint32_t>(B);   // by mesh: the largest of its triangles' (float bits)
+    float* chance = a.take<float>(B);           // by mesh: that a ray comes to it (chances_kernel)
     WB(cudaMemsetAsync(mesh_pad, 0, 4 * (size_t)B, s));
+    WB(cudaMemsetAsync(chance, 0, 4 * (size_t)B, s));
     prims_kernel<<<blocks(N, 256), 256, 0, s>>>(tlas, T, blas, B, bparent, tparent, is_root, keys, vals, boxes, used,
                                                 mesh_pad, d_state);
     shapes_kernel<<<blocks(T, 128), 128, 0, s>>>(tlas, T, blas, B, xforms, keys, mesh_pad, boxes, d_state);
@@ -921,10 +1023,10 @@ cudaError_t Build::near_trees() {
     e.first = N;
     const uint32_t all = 2 * n - trees;   // (no more than N: a binary tree of k leaves has 2k - 1 nodes here as there)
     levels_kernel<<<blocks(trees, 128), 128, 0, s>>>(node_box, cluster, trees, d_state);
-    if (scene->large) {
-        if (B) blob_area_kernel<<<blocks(B, 256), 256, 0, s>>>(blas, B, &d_state->area[0]);
-        if (all > n) near_area_kernel<<<blocks(all - n, 256), 256, 0, s>>>(e, all, &d_state->area[1]);
-    }
+    ordinary_kernel<<<blocks(T, 128), 128, 0, s>>>(tlas, T, B, keys, boxes, d_state);
+    chances_kernel<<<blocks(T, 128), 128, 0, s>>>(tlas, T, B, keys, boxes, chance, d_state);
+    blob_visits_kernel<<<blocks(N, 256), 256, 0, s>>>(tlas, T, blas, B, bparent, is_root, chance, d_state);
+    if (all > n) near_visits_kernel<<<blocks(all - n, 256), 256, 0, s>>>(e, all, tlas, blas, chance);
     WB(cudaGetLastError());
     WB(read_state());
     if (h.near_depth[0] + h.near_depth[1] <= kNearDepthLimit) total = all;
@@ -944,7 +1046,8 @@ cudaError_t Build::write_trees(float4* nodes) {
     scene->near_turn = h.turn;
     scene->near_slide = h.slide;
     scene->near_reach = h.reach + h.turn * h.world;
-    scene->near = scene->large && h.area[0] < kGoodTrees * h.area[1] ? 1u : 2u;
+    scene->visits = h.visits[0] + h.visits[1];
+    scene->near = near_level(h);
     return cudaSuccess;
 }
 

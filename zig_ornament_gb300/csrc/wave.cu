@@ -344,7 +344,7 @@ cudaError_t launch_wave_steps(const RenderLaunch& p, int shape, cudaStream_t s) 
 template <int SEM, bool FAST>
 cudaError_t launch_wave_shape(const RenderLaunch& p, const WaveConfig& c, bool count, cudaStream_t s) {
     if (count) return launch_wave_t<SEM, true, FAST, false, 0, 32>(p, s);
-    if (FAST && p.scene.near > 1u)
+    if (FAST && p.scene.near >= NEAR_WAVE)
         return c.steps == 64 ? launch_wave_steps<SEM, FAST, FAST, 64>(p, c.shape, s)
                              : launch_wave_steps<SEM, FAST, FAST, 32>(p, c.shape, s);
     return c.steps == 64 ? launch_wave_steps<SEM, FAST, false, 64>(p, c.shape, s)

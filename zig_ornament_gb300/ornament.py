@@ -741,8 +741,9 @@ class Renderer:
         return hits, visits
 
     def near_trees(self) -> int:
-        """0: the blob's trees are walked; 1: ray queries without visits take
-        the near-first trees; 2: plain renders too (orn_near_trees)."""
+        """Who walks the near-first trees: 0 nobody; 1 ray queries without visits;
+        2 also batches and render_f64; 3 also the megakernel; 4 also the
+        persistent wavefront (orn_near_trees)."""
         n = C.c_uint32()
         self._check(self._lib.orn_near_trees(self._ctx, C.byref(n)))
         return n.value
