@@ -743,42 +743,52 @@ cudaError_t launch_relmse(const float4* acc, const double* acc64, const double* 
 }
 
 // ---- host-side launchers -----------------------------------------------------
+// Blocks of kMegaBlock threads of one kernel that the device holds at once.
+// (Each launcher's is a function-local constant, as several threads may make the
+// first launch: of two ints set one after the other, one can be seen unset, and
+// they are divided by.)
+struct Residency {
+    int sms = 0;
+    uint32_t blocks = 1;
+    template <class K> explicit Residency(K* kernel) {
+        int dev = 0, per_sm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kMegaBlock, 0);
+        blocks = (uint32_t)std::max(1, std::max(1, per_sm) * sms);
+    }
+};
+
 // Persistent grid: as many blocks as fit on the device at once (never more
 // than the pixels need).
 template <int SEM, int MATH, bool COUNT, bool FAST, bool F64 = false, bool CACHE = false, bool SOBOL = false,
           bool NEAR = false, bool SPLIT = !NEAR && !CACHE>
 static cudaError_t launch_mega_tt(const RenderLaunch& p, cudaStream_t s) {
-    static int blocks_per_sm = 0, sms = 0;
-    if (blocks_per_sm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    auto* const kernel = mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR, SPLIT>;
+    static const Residency resident = [&] {
 #ifdef ORN_MEGA_CARVEOUT
         // shared-memory share of the unified L1/shared space, in percent
-        cudaFuncSetAttribute(mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR, SPLIT>,
-                             cudaFuncAttributePreferredSharedMemoryCarveout, ORN_MEGA_CARVEOUT);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, ORN_MEGA_CARVEOUT);
 #endif
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR, SPLIT>,
-                                                      kMegaBlock, 0);
-        if (blocks_per_sm < 1) blocks_per_sm = 1;
-    }
+        return Residency(kernel);
+    }();
     // A launch with fewer items than resident lanes spreads them over all
     // resident warps: a warp of two lanes runs a step's branches for two rays
     // only, and such a launch takes as long as its longest path (a frame of
     // 96 x 64 pixels, one pass, the mixed scene: 323 -> 212 us).
     RenderLaunch q = p;
     const uint64_t items = CACHE ? (uint64_t)p.pixel_count * p.cache.streams : p.pixel_count;
-    const uint32_t warps = (uint32_t)(blocks_per_sm * sms) * (kMegaBlock / 32);
+    const uint32_t warps = resident.blocks * (kMegaBlock / 32);
     // (Not the cached kernel: its training slots belong to lanes.)
     q.lanes = CACHE ? 32u : (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, (items + warps - 1) / warps));
     if (q.lanes < 32) q.shade_threshold = std::max(1, p.shade_threshold * (int)q.lanes / 32);
     const uint32_t per_block = q.lanes * (kMegaBlock / 32);
     uint32_t need = (uint32_t)((items + per_block - 1) / per_block);
-    uint32_t grid = (uint32_t)(blocks_per_sm * sms);
+    uint32_t grid = resident.blocks;
     if (need < grid) grid = need;
     cudaError_t e = cudaMemsetAsync(p.work_counter, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    mega_kernel<SEM, MATH, COUNT, FAST, F64, CACHE, SOBOL, NEAR, SPLIT><<<grid, kMegaBlock, 0, s>>>(q);
+    kernel<<<grid, kMegaBlock, 0, s>>>(q);
     return cudaGetLastError();
 }
 
@@ -839,27 +849,19 @@ cudaError_t launch_trace_rays(const SceneDev& sc, float t_min, const float* rays
         trace_rays_kernel<<<grid, 128, 0, s>>>(sc, t_min, rays, count, hits, visits, error, nullptr);
         return cudaGetLastError();
     }
-    static int blocks_per_sm = 0, sms = 0;
-    if (blocks_per_sm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, trace_near_kernel, kMegaBlock, 0);
-        if (blocks_per_sm < 1) blocks_per_sm = 1;
-    }
+    static const Residency resident(trace_near_kernel);
     cudaError_t e = cudaMemsetAsync(work, 0, 2 * sizeof(uint32_t), s);   // next ray, rays on the list
     if (e != cudaSuccess) return e;
     uint32_t* list = work + 1;
     // fewer rays than resident lanes: over all resident warps, as in launch_mega_tt
-    const uint32_t resident = (uint32_t)(blocks_per_sm * sms);
-    const uint32_t warps = resident * (kMegaBlock / 32);
+    const uint32_t warps = resident.blocks * (kMegaBlock / 32);
     const uint32_t lanes = (uint32_t)std::min<size_t>(32, (count + warps - 1) / warps);
     const uint32_t per_block = lanes * (kMegaBlock / 32);
-    const uint32_t grid = (uint32_t)std::min<size_t>(resident, (count + per_block - 1) / per_block);
+    const uint32_t grid = (uint32_t)std::min<size_t>(resident.blocks, (count + per_block - 1) / per_block);
     trace_near_kernel<<<grid, kMegaBlock, 0, s>>>(sc, t_min, rays, (uint32_t)count, hits, work, list, lanes);
     e = cudaGetLastError();
     if (e != cudaSuccess || all_safe) return e;
-    trace_rays_kernel<<<(unsigned)std::min<size_t>(blocks, (size_t)sms), 128, 0, s>>>(sc, t_min, rays, count, hits,
+    trace_rays_kernel<<<(unsigned)std::min<size_t>(blocks, (size_t)std::max(1, resident.sms)), 128, 0, s>>>(sc, t_min, rays, count, hits,
                                                                                       nullptr, error, list);
     return cudaGetLastError();
 }
